@@ -24,7 +24,7 @@ constexpr std::size_t kAlign = 256;
 std::size_t align_up(std::size_t n) { return (n + kAlign - 1) / kAlign * kAlign; }
 
 struct Workspace {
-  std::size_t xq, x4, scale, qkv, attn, ffn, w_unpack, attn_ws, total;
+  std::size_t xq, scale, qkv, attn, ffn, w_unpack, attn_ws, total;
   std::size_t attn_ws_bytes;
 };
 
@@ -50,7 +50,6 @@ Workspace carve(const b2_block_run* run_in) {
     return off;
   };
   w.xq = take(L * kmax);
-  w.x4 = take(run->tier == B2_TIER_W4A4_VIA_INT8 ? L * kmax / 2 : 0);
   w.scale = take(L * 4);
   w.qkv = take(region * 3 * D * 2);
   w.attn = take(L * D * 2);
@@ -136,7 +135,6 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
   cudaStream_t st = as_stream(stream);
   auto* base = static_cast<std::uint8_t*>(a->workspace);
   auto* xq = reinterpret_cast<std::int8_t*>(base + ws.xq);
-  auto* x4 = base + ws.x4;
   auto* scale = reinterpret_cast<float*>(base + ws.scale);
   auto* qkv = reinterpret_cast<__nv_bfloat16*>(base + ws.qkv);
   auto* attn = reinterpret_cast<__nv_bfloat16*>(base + ws.attn);
@@ -145,16 +143,15 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
   const auto* mod = static_cast<const __nv_bfloat16*>(a->mod);
   const bool a4 = run->tier == B2_TIER_W4A4_VIA_INT8;
 
-  // Quantised GEMM input of a site: INT8 activations, or INT4 activations widened to INT8 lanes.
+  // Quantised GEMM input of a site: INT8 activations, or INT4 activations in INT8 lanes (never packed: packing them and
+  // unpacking them again was three more launches, 45 us of a 1560 us block at 8484 tokens).
   const auto quant_norm = [&](const void* norm_w, const __nv_bfloat16* sc, const __nv_bfloat16* sh) -> int {
     if (!a4) return b2_rms_norm_modulate_rotate_quantize(a->x, D, norm_w, sc, sh, xq, D, scale, L, static_cast<int>(D), st, nullptr, 0);
-    if (const int rc = b2_rms_norm_modulate_convrot_quantize_int4(a->x, D, norm_w, sc, sh, x4, D / 2, scale, L, static_cast<int>(D), st)) return rc;
-    return b2_unpack_int4(x4, D / 2, xq, D, L, D, st);
+    return quantize_int4_lanes(a->x, D, norm_w, sc, sh, xq, D, scale, L, static_cast<int>(D), st);
   };
   const auto quant_plain = [&](const __nv_bfloat16* in, std::int64_t k) -> int {
     if (!a4) return b2_rotate_quantize(in, k, xq, k, scale, L, static_cast<int>(k), st);
-    if (const int rc = b2_convrot_quantize_int4(in, k, x4, k / 2, scale, L, static_cast<int>(k), st)) return rc;
-    return b2_unpack_int4(x4, k / 2, xq, k, L, k, st);
+    return quantize_int4_lanes(in, k, nullptr, nullptr, nullptr, xq, k, scale, L, static_cast<int>(k), st);
   };
   // One linear site with its epilogue (0 plain, 1 gated residual with gate `aux`, 2 SiTU-GLU) under the run's tier. The
   // grouped 4-bit tier goes through b2_w4a8_gemm, which decodes inside the GEMM where the weight's format allows and

@@ -36,6 +36,26 @@ int attn_status_clear();
 // Test hooks of the GEMM kernel's bounded waits: the limit in nanoseconds (0 = leave it) and the "skip one stage" switch.
 int gemm_debug_set(unsigned long long wait_limit_ns, int skip_stage);
 
+// Fills the SiTU factor tables of the current device once (on `stream`, which it synchronises the first time); a no-op
+// afterwards. For callers that are about to capture: inside a capture every SiTU-GLU launch would bring a fill along.
+int prepare_situ_tables(cudaStream_t stream);
+
+// Key and value rows of an attention call beyond its k and v views. Rows [own0, own0 + q rows) of the views are the run's
+// own; the rows before and after them are read from slot[0] and slot[1] (bf16 rows k | v, 16-byte aligned, slot_ld
+// elements apart). tap, when set, receives a copy of the own k | v rows [q rows, 2 heads 128].
+struct AttentionRows {
+  const void* slot[2];
+  std::int64_t slot_ld, own0;
+  void* tap;
+};
+int attention_rows(const b2_attention_options* o, const b2_view3* q, const b2_view3* k, const b2_view3* v, const b2_view3* out,
+                   const std::int32_t* cu_q, const std::int32_t* cu_k, int batch, int max_seqlen, float scale, void* workspace,
+                   std::size_t workspace_bytes, void* stream, const b2_qk_norm_rope* norm_rope, const AttentionRows& rows);
+
+// The INT4 quantiser (with its norm + modulate prologue when norm_weight is given), its codes left in INT8 lanes [m, k].
+int quantize_int4_lanes(const void* x, std::int64_t ldx, const void* norm_weight, const void* mod_scale, const void* mod_shift,
+                        std::int8_t* q, std::int64_t ldq, float* scale, std::int64_t m, int k, void* stream);
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

@@ -46,6 +46,7 @@ struct Args {
   const __nv_bfloat16* mod_shift;
   __nv_bfloat16* y;
   std::int64_t ldy;
+  int lanes;     // INT4 only: leave the codes in INT8 lanes instead of packing two to a byte
   float factor;  // float(m) / float(m * k)
   int bw;        // torch's threads per row for this (m, k)
   // Column-chunked input (0 = off): columns [i * chunk_w, (i + 1) * chunk_w) of every row live in chunk i, a [m, chunk_w]
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kPairs == 1 ? 384 : 512, kPairs == 1 ? 2 : 1) 
       for (int gi = 0; gi < 2; ++gi) {
         const int g = 2 * (half_id + p * halves) + gi;
         if (g >= groups) continue;
-        if constexpr (kInt4) {
+        if (kInt4 && a.lanes == 0) {
           const u32 w[4] = {bytes[gi].x, bytes[gi].y, bytes[gi].z, bytes[gi].w};
           u32 out[2];
 #pragma unroll
@@ -579,31 +580,45 @@ int check_norm(const char* op, const void* w, const void* sc, const void* sh, st
 
 // ------------------------------------------------------------------------------------------------ int4 helpers
 
-// 32 values per thread: 16 packed bytes in, 32 bytes out. Signed nibbles, even column in the low nibble.
-__global__ void unpack_int4_kernel(const std::uint8_t* packed, std::int64_t ldp, std::int8_t* out, std::int64_t ldo,
-                                   std::int64_t rows, int chunks_per_row) {
-  const std::int64_t total = rows * chunks_per_row;
-  for (std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
-    const std::int64_t r = i / chunks_per_row;
-    const int c = static_cast<int>(i % chunks_per_row);
-    const uint4 in = *reinterpret_cast<const uint4*>(packed + r * ldp + 16 * c);
-    const std::uint32_t w[4] = {in.x, in.y, in.z, in.w};
-    std::uint32_t o[8];
+constexpr int kUnpackUnroll = 4;
+// 16 values per thread: 8 packed bytes in, 16 bytes out. Signed nibbles, even column in the low nibble. kFlat: contiguous
+// rows, no row arithmetic (whose 64-bit division, with two dependent loads in flight per thread, held the kernel at half of
+// the memory rate).
+template <bool kFlat>
+__global__ void __launch_bounds__(256) unpack_int4_kernel(const std::uint8_t* packed, std::int64_t ldp, std::int8_t* out,
+                                                          std::int64_t ldo, std::int64_t items, unsigned per_row) {
+  const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
+  for (std::int64_t i0 = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < items; i0 += kUnpackUnroll * stride) {
+    uint2 in[kUnpackUnroll];
+    std::int64_t at[kUnpackUnroll];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      // Sign-extend each nibble into its own byte: shift to the top of the byte, arithmetic shift back (per byte).
-      const std::uint32_t lo = (w[j] << 4) & 0xF0F0F0F0u, hi = w[j] & 0xF0F0F0F0u;
-      // bytes of lo/hi hold nibble << 4; __vshr-like per-byte arithmetic shift via sign mask.
-      const std::uint32_t lo_s = ((lo >> 4) & 0x0F0F0F0Fu) | (((lo >> 7) & 0x01010101u) * 0xF0u);
-      const std::uint32_t hi_s = ((hi >> 4) & 0x0F0F0F0Fu) | (((hi >> 7) & 0x01010101u) * 0xF0u);
-      // interleave: out bytes = lo0, hi0, lo1, hi1 | lo2, hi2, lo3, hi3
-      o[2 * j] = __byte_perm(lo_s, hi_s, 0x5140);
-      o[2 * j + 1] = __byte_perm(lo_s, hi_s, 0x7362);
+    for (int u = 0; u < kUnpackUnroll; ++u) {
+      const std::int64_t i = i0 + u * stride;
+      if (i >= items) break;
+      if constexpr (kFlat) {
+        in[u] = __ldcs(reinterpret_cast<const uint2*>(packed) + i), at[u] = 16 * i;
+      } else {
+        const std::int64_t r = i / per_row, c = i - r * per_row;
+        in[u] = __ldcs(reinterpret_cast<const uint2*>(packed + r * ldp) + c), at[u] = r * ldo + 16 * c;
+      }
     }
-    uint4* dst = reinterpret_cast<uint4*>(out + r * ldo + 32 * c);
-    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+#pragma unroll
+    for (int u = 0; u < kUnpackUnroll; ++u) {
+      if (i0 + u * stride >= items) break;
+      const u32 w[2] = {in[u].x, in[u].y};
+      u32 o[4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        // Each nibble at the top of its byte, then an arithmetic shift right by four within the byte.
+        const u32 lo = (w[j] << 4) & 0xF0F0F0F0u, hi = w[j] & 0xF0F0F0F0u;
+        const u32 lo_s = ((lo >> 4) & 0x0F0F0F0Fu) | (((lo >> 7) & 0x01010101u) * 0xF0u);
+        const u32 hi_s = ((hi >> 4) & 0x0F0F0F0Fu) | (((hi >> 7) & 0x01010101u) * 0xF0u);
+        // out bytes = lo0, hi0, lo1, hi1 | lo2, hi2, lo3, hi3
+        o[2 * j] = __byte_perm(lo_s, hi_s, 0x5140);
+        o[2 * j + 1] = __byte_perm(lo_s, hi_s, 0x7362);
+      }
+      *reinterpret_cast<uint4*>(out + at[u]) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
   }
 }
 
@@ -619,40 +634,88 @@ __device__ __forceinline__ float e4m3_bits_to_float(std::uint32_t b) {
 // Raised (OR 1) by a decode that met a NaN or negative group scale and was given no word of the caller's.
 __device__ unsigned g_w4_invalid = 0;
 
+// Four 4-bit codes -> the bytes of the 16-entry table `t` (entry i in byte i % 4 of word i / 4): two byte permutes pick among
+// entries 0..7 and 8..15 by the low three bits of each code (s1), a third takes the right one by the code's top bit (s2).
+__device__ __forceinline__ u32 expand4(u32 s1, u32 s2, const uint4& t) {
+  return __byte_perm(__byte_perm(t.x, t.y, s1), __byte_perm(t.z, t.w, s1), s2);
+}
+
+constexpr int kDecodeUnroll = 4;
+
 // 16 columns per thread (8 packed bytes): level * group scale, rne, clamp to +-127. A group whose scale is NaN or
-// negative decodes to zeros and raises *invalid (src/kernels/quant/w4a8_decode.cu:57-62).
-__global__ void decode_grouped_kernel(const std::uint8_t* packed, const void* s_rel, int scale_kind, const float* codebook,
-                                      std::int64_t rows, std::int64_t k, int group, std::int8_t* out, unsigned* invalid) {
+// negative decodes to zeros and raises *invalid (src/kernels/quant/w4a8_decode.cu:57-62). Rows are contiguous and hold
+// whole groups, so everything is indexed by the flat column index; `shift` is log2(group), or -1 for other group sizes.
+// kTable (e4m3 scales): the 16 decoded values of every scale byte are tabulated once per block in shared memory, and a
+// thread expands its codes with byte permutes. Computing each value from its code and the row arithmetic (64-bit
+// divisions) held the kernel at 2.2 TB/s (56 us for a 24576 x 3072 weight); what bounds it now is HBM.
+template <bool kTable>
+__global__ void __launch_bounds__(256) decode_grouped_kernel(const std::uint8_t* packed, const void* s_rel, const float* codebook,
+                                                             std::int64_t items, int group, int shift, std::int8_t* out,
+                                                             unsigned* invalid) {
   __shared__ float s_cb[16];
+  __shared__ uint4 s_table[kTable ? 256 : 1];
   if (threadIdx.x < 16) s_cb[threadIdx.x] = codebook != nullptr ? codebook[threadIdx.x] : static_cast<float>(threadIdx.x) - 8.0f;
   __syncthreads();
-  const std::int64_t per_row = k / 16, total = rows * per_row, groups = k / group;
-  for (std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
-    const std::int64_t r = i / per_row, c0 = (i % per_row) * 16;
-    const std::int64_t gi = r * groups + c0 / group;
-    float s;
-    if (scale_kind == 0) s = e4m3_bits_to_float(static_cast<const std::uint8_t*>(s_rel)[gi]);
-    else s = __half2float(__ushort_as_half(static_cast<const unsigned short*>(s_rel)[gi]));
-    const bool ok = !(isnan(s) || s < 0.0f);
-    const uint2 in = *reinterpret_cast<const uint2*>(packed + r * (k / 2) + c0 / 2);
-    const std::uint32_t w[2] = {in.x, in.y};
-    std::uint32_t o[4];
+  const auto decoded = [&](u32 code, float s) {
+    return static_cast<u32>(static_cast<int>(fminf(127.f, fmaxf(-127.f, rintf(fmul(s_cb[code], s)))))) & 0xFFu;
+  };
+  if constexpr (kTable) {
+    const float s = e4m3_bits_to_float(threadIdx.x);
+    u32 t[4] = {0u, 0u, 0u, 0u};
+    if (!(isnan(s) || s < 0.0f)) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      std::uint32_t word = 0;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int col = 4 * j + b;
-        const std::uint32_t code = (w[col / 8] >> (4 * (col % 8))) & 0xF;
-        const float vq = fminf(127.f, fmaxf(-127.f, rintf(fmul(s_cb[code], s))));
-        word |= (static_cast<std::uint32_t>(static_cast<int>(vq)) & 0xFF) << (8 * b);
-      }
-      o[j] = ok ? word : 0u;
+      for (u32 c = 0; c < 16; ++c) t[c >> 2] |= decoded(c, s) << (8 * (c & 3));
     }
-    *reinterpret_cast<uint4*>(out + r * k + c0) = make_uint4(o[0], o[1], o[2], o[3]);
-    if (!ok) atomicOr(invalid, 1u);
+    s_table[threadIdx.x] = make_uint4(t[0], t[1], t[2], t[3]);
+    __syncthreads();
   }
+  const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
+  bool bad = false;
+  for (std::int64_t i0 = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < items; i0 += kDecodeUnroll * stride) {
+    uint2 in[kDecodeUnroll];
+    u32 sb[kDecodeUnroll];
+#pragma unroll
+    for (int u = 0; u < kDecodeUnroll; ++u) {
+      const std::int64_t i = i0 + u * stride;
+      if (i < items) {
+        const std::int64_t g = shift >= 0 ? (i << 4) >> shift : (i << 4) / group;
+        in[u] = __ldcs(reinterpret_cast<const uint2*>(packed) + i);
+        sb[u] = kTable ? static_cast<u32>(static_cast<const std::uint8_t*>(s_rel)[g]) : static_cast<u32>(static_cast<const unsigned short*>(s_rel)[g]);
+      } else {
+        in[u] = make_uint2(0u, 0u), sb[u] = 0u;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kDecodeUnroll; ++u) {
+      const std::int64_t i = i0 + u * stride;
+      if (i >= items) break;
+      const u32 w[2] = {in[u].x, in[u].y};
+      u32 o[4];
+      if constexpr (kTable) {
+        bad |= (sb[u] & 0x7Fu) == 0x7Fu || sb[u] > 0x80u;  // NaN, or the sign bit over a non-zero magnitude
+        const uint4 t = s_table[sb[u]];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const u32 s1 = w[j] & 0x77777777u, s2 = ((w[j] >> 1) & 0x44444444u) | 0x32103210u;
+          o[2 * j] = expand4(s1, s2, t);
+          o[2 * j + 1] = expand4(s1 >> 16, s2 >> 16, t);
+        }
+      } else {
+        const float s = __half2float(__ushort_as_half(static_cast<unsigned short>(sb[u])));
+        const bool ok = !(isnan(s) || s < 0.0f);
+        bad |= !ok;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          u32 word = 0;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) word |= decoded((w[j >> 1] >> (16 * (j & 1) + 4 * b)) & 0xFu, s) << (8 * b);
+          o[j] = ok ? word : 0u;
+        }
+      }
+      reinterpret_cast<uint4*>(out)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+  if (bad) atomicOr(invalid, 1u);
 }
 
 }  // namespace
@@ -766,6 +829,26 @@ int b2_rms_norm_modulate_convrot_quantize_int4(const void* x, int64_t ldx, const
   return launch<true, true>(op, a, m, as_stream(stream));
 }
 
+}  // extern "C"
+
+int b2::quantize_int4_lanes(const void* x, std::int64_t ldx, const void* norm_weight, const void* mod_scale, const void* mod_shift,
+                            std::int8_t* q, std::int64_t ldq, float* scale, std::int64_t m, int k, void* stream) {
+  constexpr const char* op = "convrot_quantize_int4";
+  if (const int rc = check_common(op, x, ldx, q, ldq, scale, m, k, false)) return rc;
+  Args a{};
+  a.x = static_cast<const __nv_bfloat16*>(x), a.ldx = ldx, a.q = q, a.ldq = ldq, a.scale = scale, a.k = k, a.lanes = 1;
+  if (norm_weight == nullptr) return m == 0 ? B2_OK : launch<false, true>(op, a, m, as_stream(stream));
+  if (const int rc = check_norm(op, norm_weight, mod_scale, mod_shift, m, k, &a.bw)) return rc;
+  if (m == 0) return B2_OK;
+  a.weight = static_cast<const __nv_bfloat16*>(norm_weight);
+  a.mod_scale = static_cast<const __nv_bfloat16*>(mod_scale);
+  a.mod_shift = static_cast<const __nv_bfloat16*>(mod_shift);
+  a.factor = static_cast<float>(m) / static_cast<float>(m * k);
+  return launch<true, true>(op, a, m, as_stream(stream));
+}
+
+extern "C" {
+
 int b2_unpack_int4(const void* packed, int64_t ldp, int8_t* out, int64_t ldo, int64_t rows, int64_t k, void* stream) {
   constexpr const char* op = "unpack_int4";
   if (rows < 0 || k <= 0 || k % 32 != 0) return fail_invalid(op, "k must be a positive multiple of 32");
@@ -774,10 +857,10 @@ int b2_unpack_int4(const void* packed, int64_t ldp, int8_t* out, int64_t ldo, in
       ldo % 16 != 0 || ldp < k / 2 || ldo < k) {
     return fail_invalid(op, "needs 16-byte aligned rows (ldp % 16 == 0, ldo % 16 == 0)");
   }
-  const int chunks = static_cast<int>(k / 32);
-  const std::int64_t total = rows * chunks;
-  const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((total + 255) / 256, 148 * 16));
-  unpack_int4_kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const std::uint8_t*>(packed), ldp, out, ldo, rows, chunks);
+  const std::int64_t total = rows * (k / 16);
+  const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((total + 256 * kUnpackUnroll - 1) / (256 * kUnpackUnroll), sm_count() * 8LL));
+  const auto kernel = ldp == k / 2 && ldo == k ? unpack_int4_kernel<true> : unpack_int4_kernel<false>;
+  kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const std::uint8_t*>(packed), ldp, static_cast<std::int8_t*>(out), ldo, total, static_cast<unsigned>(k / 16));
   return check_launch(op);
 }
 
@@ -799,9 +882,14 @@ int b2_decode_grouped_int8(const void* packed, const void* s_rel, int scale_kind
     invalid = static_cast<unsigned*>(word);
   }
   const std::int64_t total = rows * (k / 16);
-  const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((total + 255) / 256, 148 * 16));
-  decode_grouped_kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const std::uint8_t*>(packed), s_rel, scale_kind,
-                                                              codebook, rows, k, group, out, invalid);
+  const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((total + 256 * kDecodeUnroll - 1) / (256 * kDecodeUnroll), sm_count() * 8LL));
+  int shift = -1;
+  if ((group & (group - 1)) == 0) {
+    for (shift = 4; (1 << shift) < group; ++shift) {
+    }
+  }
+  const auto kernel = scale_kind == 0 ? decode_grouped_kernel<true> : decode_grouped_kernel<false>;
+  kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const std::uint8_t*>(packed), s_rel, codebook, total, group, shift, out, invalid);
   return check_launch(op);
 }
 

@@ -1,0 +1,88 @@
+"""Kernel variants chosen by size, alignment or option, each at the sizes where its choice or its edges lie, held to the
+CPU oracle or to the bits of the form it stands in for."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle_lib as orc
+from owoinfer_b200 import synth
+
+pytestmark = pytest.mark.gpu
+D, H = 3072, 24
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from owoinfer_b200 import ops as o
+    yield o
+    torch.cuda.synchronize()
+    assert o.kernel_status() == (0, 0)
+
+
+def bits(t):
+    return t.contiguous().view(torch.int16).cpu().numpy().view(np.uint16)
+
+
+# One item; a remainder of the 1024-item step of a block; more items than one step of the whole grid takes.
+@pytest.mark.parametrize("rows,k,group", [(1, 32, 16), (3, 96, 32), (37, 3072, 64), (5, 3072, 48), (1300, 12288, 128)])
+def test_four_bit_weights_to_int8(ops, rows, k, group):
+    rng = np.random.default_rng(rows)
+    packed = rng.integers(0, 256, (rows, k // 2), dtype=np.uint8)
+    dp = torch.from_numpy(packed).cuda()
+    assert np.array_equal(ops.unpack_int4(dp).cpu().numpy(), orc.unpack_int4(packed))
+    if k % 32 == 0 and rows > 1:  # padded rows on both sides
+        wide, out = torch.zeros((rows, k // 2 + 16), dtype=torch.uint8, device="cuda"), torch.full((rows, k + 16), 99, dtype=torch.int8, device="cuda")
+        wide[:, :k // 2] = dp
+        ops.unpack_int4(wide[:, :k // 2], out=out[:, :k])
+        assert np.array_equal(out[:, :k].cpu().numpy(), orc.unpack_int4(packed)) and (out[:, k:] == 99).all()
+    e4m3 = rng.integers(0x18, 0x58, (rows, k // group), dtype=np.uint8)
+    fp16 = (rng.random((rows, k // group)).astype(np.float32) * 12 + 0.01).astype(np.float16).view(np.uint16)
+    cb = rng.normal(0, 4, 16).astype(np.float32)
+    for scales, dev in ((e4m3, torch.from_numpy(e4m3).cuda()), (fp16, torch.from_numpy(fp16.view(np.int16)).cuda())):
+        want = orc.decode_grouped_int8(packed, scales, group)
+        assert np.array_equal(ops.decode_grouped_int8(dp, dev, group).cpu().numpy(), want)
+        want = orc.decode_grouped_int8(packed, scales, group, cb)
+        assert np.array_equal(ops.decode_grouped_int8(dp, dev, group, torch.from_numpy(cb).cuda()).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("slot,n0,n1", [(7, 65, 1), (128, 200, 333)])
+def test_tap_and_slots_read_in_place_equal_the_copied_forms(ops, slot, n0, n1):
+    """k | v rows tapped by the pass that quantises them, and slot rows read where they lie, against the copies that rows
+    without 16-byte alignment take, and against the separate QK-norm + RoPE."""
+    F = 512
+    w = synth.block_weights(D, F, 31)
+    bw = ops.BlockWeights(w["norm1"], w["norm2"], w["q_norm"], w["k_norm"], w["qkv"], w["o"], w["up_gate"], w["down"])
+    mod, L = synth.modulation(D, 4), n0 + n1
+    x0 = synth.activations(L, D, 9)
+    rope = ops.moss_rope_table(1, 1, L - 1)
+    cu = synth.cu_seqlens([n0, n1])
+
+    def run(**kw):
+        r = ops.block_run(L, cu, max(n0, n1) + kw.pop("extra", 0), D=D, F=F, **kw)
+        ws = torch.empty(ops.block_quant_workspace_bytes(r), dtype=torch.uint8, device="cuda")
+        x = x0.clone()
+        ops.run_block_quant(bw, ops.block_buffers(x, mod, rope, ws), r)
+        torch.cuda.synchronize()
+        return bits(x)
+
+    flat = torch.zeros(L * 2 * D + 8, dtype=torch.bfloat16, device="cuda")
+    taps = [flat[o:o + L * 2 * D].view(L, 2 * D) for o in (0, 4)]      # the second one only 8-byte aligned
+    seen = []
+    for tap in taps:
+        tap.zero_()
+        seen.append((run(kv_tap=tap), bits(tap)))
+    plain = run()
+    assert all(np.array_equal(y, plain) for y, _ in seen) and np.array_equal(seen[0][1], seen[1][1]) and seen[0][1].any()
+
+    kv = torch.randn(slot * 2 * D + 8, device="cuda", generator=torch.Generator("cuda").manual_seed(slot)).to(torch.bfloat16)
+    odd = torch.empty_like(kv)
+    odd[4:4 + slot * 2 * D] = kv[:slot * 2 * D]
+    aligned, shifted = kv[:slot * 2 * D].view(slot, 2 * D), odd[4:4 + slot * 2 * D].view(slot, 2 * D)
+    both = dict(slot_rows=slot, cu_seqlens_k=synth.cu_seqlens([slot + n0, n1 + slot]), k0=0, k1=L + 2 * slot, extra=slot)
+    want = run(slot_kv=(shifted, shifted), **both)
+    assert np.array_equal(run(slot_kv=(aligned, aligned), **both), want)
+    assert np.array_equal(run(slot_kv=(aligned, aligned), fused_norm_rope=0, **both), want)
+    one = dict(slot_rows=slot, cu_seqlens_k=synth.cu_seqlens([n0, n1 + slot]), k0=slot, k1=L + 2 * slot, extra=slot)
+    assert np.array_equal(run(slot_kv=(None, aligned), **one), run(slot_kv=(None, shifted), **one))
