@@ -263,6 +263,12 @@ struct PrepArgs {
   const __nv_bfloat16* table;
   std::int64_t table_row;
   float norm_factor;
+  // Keys and values that live elsewhere (a block run over cached reference rows): key rows [own0, own1) are rows of k / v,
+  // the rows before and after them rows of slot[0] and slot[1] (k | v side by side, slot_ld elements apart). Without slots
+  // own0 = 0 and own1 is past every row.
+  const __nv_bfloat16* slot[2];
+  std::int64_t slot_ld, own0, own1;
+  __nv_bfloat16* tap;  // when set: a copy of the own rows' k | v, [own1 - own0, 2 heads 128]
   // outputs
   std::int8_t* q_i8;
   std::int8_t* k_i8;
@@ -275,6 +281,16 @@ struct PrepArgs {
   float* part_sum;
   float* part_amax;
 };
+
+// Where head 0 of key row `tok` starts in the K and V rows.
+__device__ __forceinline__ void kv_rows(const PrepArgs& p, std::int64_t tok, const __nv_bfloat16*& k, const __nv_bfloat16*& v) {
+  if (tok >= p.own0 && tok < p.own1) {
+    k = p.k + tok * p.k_row, v = p.v + tok * p.v_row;
+  } else {
+    k = (tok < p.own0 ? p.slot[0] + tok * p.slot_ld : p.slot[1] + (tok - p.own1) * p.slot_ld);
+    v = k + static_cast<std::int64_t>(p.heads) * kHeadDim;
+  }
+}
 
 // Packed bf16 pairs: a * b and a + b, each result rounded once to bf16. For bf16 operands these equal the fp32 operation
 // followed by a rounding to bf16 (the fp32 product of two bf16 values is exact; an fp32 sum of two bf16 values is either
@@ -405,8 +421,10 @@ __global__ void __launch_bounds__(256) stats_kernel(const PrepArgs p) {
       const int t = t0 + 16 * u;
       const std::int64_t tok = static_cast<std::int64_t>(start) + t;
       if (t < t_end) {
-        kr[u] = *reinterpret_cast<const uint4*>(p.k + tok * p.k_row + h * p.k_head + lane * 8);
-        vr[u] = *reinterpret_cast<const uint4*>(p.v + tok * p.v_row + h * p.v_head + lane * 8);
+        const __nv_bfloat16 *k_at, *v_at;
+        kv_rows(p, tok, k_at, v_at);
+        kr[u] = *reinterpret_cast<const uint4*>(k_at + h * p.k_head + lane * 8);
+        vr[u] = *reinterpret_cast<const uint4*>(v_at + h * p.v_head + lane * 8);
       } else {
         kr[u] = vr[u] = make_uint4(0, 0, 0, 0);  // +0 leaves the sum and the maximum as they are
       }
@@ -505,8 +523,21 @@ __global__ void __launch_bounds__(256) quant_kv_kernel(const PrepArgs p) {
     tok[i] = static_cast<std::int64_t>(start) + t;
     kr[i] = vr[i] = make_uint4(0, 0, 0, 0);
     if (valid[i]) {
-      kr[i] = *reinterpret_cast<const uint4*>(p.k + tok[i] * p.k_row + h * p.k_head + lane * 8);
-      vr[i] = *reinterpret_cast<const uint4*>(p.v + tok[i] * p.v_row + h * p.v_head + lane * 8);
+      const __nv_bfloat16 *k_at, *v_at;
+      kv_rows(p, tok[i], k_at, v_at);
+      kr[i] = *reinterpret_cast<const uint4*>(k_at + h * p.k_head + lane * 8);
+      vr[i] = *reinterpret_cast<const uint4*>(v_at + h * p.v_head + lane * 8);
+    }
+  }
+  if (p.tap != nullptr) {
+    // The rows pass through these registers anyway: a copy of the whole k | v matrix of its own would read them once more.
+    const std::int64_t width = static_cast<std::int64_t>(p.heads) * kHeadDim;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (!valid[i] || tok[i] < p.own0 || tok[i] >= p.own1) continue;
+      __nv_bfloat16* at = p.tap + (tok[i] - p.own0) * 2 * width + h * kHeadDim + lane * 8;
+      __stcs(reinterpret_cast<uint4*>(at), kr[i]);
+      __stcs(reinterpret_cast<uint4*>(at + width), vr[i]);
     }
   }
   float mean[8], recp[8];
@@ -1262,7 +1293,8 @@ struct ScoreDump {
 int attention_impl(const char* op, const b2_attention_options* o, const b2_view3* q, const b2_view3* k, const b2_view3* v,
                    const b2_view3* out, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int batch,
                    int max_seqlen, float scale, void* workspace, size_t workspace_bytes, void* stream,
-                   const b2_qk_norm_rope* norm_rope, const ScoreDump* dump, bool prepass_only = false) {
+                   const b2_qk_norm_rope* norm_rope, const ScoreDump* dump, bool prepass_only = false,
+                   const AttentionRows* rows = nullptr) {
   if (o == nullptr) return fail_invalid(op, "null options");
   if (const int rc = check_view(op, q, "q")) return rc;
   if (const int rc = check_view(op, k, "k")) return rc;
@@ -1299,7 +1331,7 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
         norm_rope->table_ld % 8 != 0 || norm_rope->table_ld < kHeadDim) {
       return fail_invalid(op, "norm_rope: q_norm, k_norm and table must be 16-byte aligned bf16 device tensors");
     }
-    if (cu_seqlens_k != cu_seqlens_q || k->row_stride != q->row_stride || total_k != total_q) {
+    if (rows == nullptr && (cu_seqlens_k != cu_seqlens_q || k->row_stride != q->row_stride || total_k != total_q)) {
       return fail_invalid(op, "norm_rope needs one cu_seqlens tensor and q and k rows of one stride");
     }
   }
@@ -1330,15 +1362,23 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   p.v_recp = reinterpret_cast<float*>(base + l.v_recp);
   p.part_sum = reinterpret_cast<float*>(base + l.part_sum);
   p.part_amax = reinterpret_cast<float*>(base + l.part_amax);
+  p.own1 = total_k;
+  if (rows != nullptr) {
+    p.slot[0] = static_cast<const __nv_bfloat16*>(rows->slot[0]), p.slot[1] = static_cast<const __nv_bfloat16*>(rows->slot[1]);
+    p.slot_ld = rows->slot_ld, p.own0 = rows->own0, p.own1 = rows->own0 + total_q;
+    p.tap = static_cast<__nv_bfloat16*>(rows->tap);
+  }
   const dim3 stats_grid(l.chunks, static_cast<unsigned>(heads), batch);
   if (norm_rope != nullptr) {
-    const std::int64_t rows = total_q * heads;
+    const std::int64_t norm_rows = total_q * heads;
     p.q_norm = static_cast<const __nv_bfloat16*>(norm_rope->q_norm);
     p.k_norm = static_cast<const __nv_bfloat16*>(norm_rope->k_norm);
     p.table = static_cast<const __nv_bfloat16*>(norm_rope->table);
     p.table_row = norm_rope->table_ld;
-    p.norm_factor = static_cast<float>(rows) / static_cast<float>(rows * kHeadDim);
-    norm_rope_quant_q_kernel<<<dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st>>>(p);
+    p.norm_factor = static_cast<float>(norm_rows) / static_cast<float>(norm_rows * kHeadDim);
+    PrepArgs own = p;  // queries and the key rows of the same tokens
+    own.cu = cu_seqlens_q, own.k = p.k + p.own0 * p.k_row;
+    norm_rope_quant_q_kernel<<<dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st>>>(own);
     if (const int rc = check_launch(op)) return rc;
   }
   stats_kernel<<<stats_grid, 256, 0, st>>>(p);
@@ -1390,6 +1430,17 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   return check_launch(op);
 }
 }  // namespace
+}  // extern "C"
+
+// b2_attention_q8 of a block run whose keys are partly cached rows, or whose k | v rows are to be copied out.
+int b2::attention_rows(const b2_attention_options* o, const b2_view3* q, const b2_view3* k, const b2_view3* v, const b2_view3* out,
+                       const std::int32_t* cu_q, const std::int32_t* cu_k, int batch, int max_seqlen, float scale, void* workspace,
+                       std::size_t workspace_bytes, void* stream, const b2_qk_norm_rope* norm_rope, const AttentionRows& rows) {
+  return attention_impl("attention_q8", o, q, k, v, out, cu_q, cu_k, batch, max_seqlen, scale, workspace, workspace_bytes, stream,
+                        norm_rope, nullptr, false, &rows);
+}
+
+extern "C" {
 
 int b2_attention_q8(const b2_attention_options* o, const b2_view3* q, const b2_view3* k, const b2_view3* v,
                     const b2_view3* out, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int batch,

@@ -177,18 +177,25 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
   if (const int rc = quant_norm(w->norm1, mod + 1 * D, mod + 0 * D)) return rc;
   if (const int rc = site(w->qkv, 3 * D, D, 0, nullptr, own, 3 * D)) return rc;
 
-  // Attention. QK-norm + RoPE inside the pre-pass from 3072 tokens on (same bits either way); as their own kernel when
-  // the keys are not the run's own rows alone or the rows are tapped after them.
-  const bool plain = slot == 0 && run->kv_tap == nullptr;
-  // Automatic = the pre-pass at every size: the two routes give the same bits, and on this part the fused one is the faster
-  // from 2 x 320 tokens (167 against 173 us per block) to 2 x 8192 (the reference's sm_89 measurements put the switch at
-  // 3072 rows, dit_block_quant.cpp:32-35).
-  const bool fused = plain && (run->fused_norm_rope < 0 || run->fused_norm_rope != 0);
+  // Attention. QK-norm + RoPE inside the pre-pass at every size: the two routes give the same bits, and on this part the
+  // fused one is the faster from 2 x 320 tokens (167 against 173 us per block) to 2 x 8192 (the reference's sm_89
+  // measurements put the switch at 3072 rows, dit_block_quant.cpp:32-35). Cached key and value rows are read where they lie
+  // and tapped rows leave with the pass that quantises them, as long as their rows allow 16-byte accesses: at 4378 + 4106
+  // tokens over 4096 reference rows the copies into the QKV matrix took 107 us of a 2095 us block, a tap of 4096 rows 53 us
+  // of 808 us. Rows that do not are copied first, and a run that ends at the tap has no pre-pass.
+  const std::size_t kv_bytes = static_cast<std::size_t>(2 * D) * sizeof(__nv_bfloat16), row_bytes = static_cast<std::size_t>(3 * D) * sizeof(__nv_bfloat16);
+  const std::int64_t slot_ld = run->slot_kv_ld > 0 ? run->slot_kv_ld : 2 * D;
+  const bool reads[2] = {slot > 0 && run->k0 < slot, slot > 0 && run->k1 > slot + L};
+  bool direct = run->kv_tap == nullptr || (run->tap_only == 0 && slot == 0);
+  direct = direct && aligned_to(run->kv_tap, 16) && slot_ld % 8 == 0;
+  for (int s2 = 0; s2 < 2; ++s2) direct = direct && (!reads[s2] || aligned_to(run->slot_kv[s2], 16));
+  // (Key rows that leave out some of the run's own tokens keep the copies: the pre-pass counts own rows from its queries.)
+  if (slot > 0) direct = direct && run->k0 <= slot && run->k1 >= slot + L;
+  const bool fused = direct && run->fused_norm_rope != 0;
   if (!fused) {
     if (const int rc = b2_qk_norm_rope_moss(own, 3 * D, L, run->heads, w->q_norm, w->k_norm, a->rope, 128, st)) return rc;
   }
-  const std::size_t kv_bytes = static_cast<std::size_t>(2 * D) * sizeof(__nv_bfloat16), row_bytes = static_cast<std::size_t>(3 * D) * sizeof(__nv_bfloat16);
-  if (run->kv_tap != nullptr) {
+  if (run->kv_tap != nullptr && !direct) {
     // tap_reference_kv: the k | v columns of every row, contiguous.
     if (const cudaError_t e = cudaMemcpy2DAsync(run->kv_tap, kv_bytes, own + D, row_bytes, kv_bytes, static_cast<std::size_t>(L), cudaMemcpyDeviceToDevice, st); e != cudaSuccess) {
       return fail_cuda(op, e);
@@ -197,19 +204,24 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
   }
   std::int64_t k0 = 0, k_rows = L;
   const std::int32_t* cu_k = run->cu_seqlens;
+  AttentionRows rows{};
   if (slot > 0) {
     // The cached keys and values into the k | v columns of the slots the key rows reach (moss_dit.cpp:1441-1452).
     for (int s2 = 0; s2 < 2; ++s2) {
-      const bool read = s2 == 0 ? run->k0 < slot : run->k1 > slot + L;
-      if (!read) continue;
+      if (!reads[s2] || direct) continue;
       __nv_bfloat16* dst = qkv + (s2 == 0 ? 0 : slot + L) * 3 * D + D;
-      const std::size_t src_pitch = run->slot_kv_ld > 0 ? static_cast<std::size_t>(run->slot_kv_ld) * sizeof(__nv_bfloat16) : kv_bytes;
-      if (const cudaError_t e = cudaMemcpy2DAsync(dst, row_bytes, run->slot_kv[s2], src_pitch, kv_bytes, static_cast<std::size_t>(slot), cudaMemcpyDeviceToDevice, st); e != cudaSuccess) {
+      if (const cudaError_t e = cudaMemcpy2DAsync(dst, row_bytes, run->slot_kv[s2], static_cast<std::size_t>(slot_ld) * sizeof(__nv_bfloat16), kv_bytes, static_cast<std::size_t>(slot), cudaMemcpyDeviceToDevice, st); e != cudaSuccess) {
         return fail_cuda(op, e);
       }
     }
     k0 = run->k0, k_rows = run->k1 - run->k0, cu_k = run->cu_seqlens_k;
+    if (direct) {
+      rows.own0 = slot - k0, rows.slot_ld = slot_ld;
+      if (reads[0]) rows.slot[0] = static_cast<const __nv_bfloat16*>(run->slot_kv[0]) + k0 * slot_ld;
+      if (reads[1]) rows.slot[1] = run->slot_kv[1];
+    }
   }
+  if (direct) rows.tap = run->kv_tap;
   const b2_view3 vq{own, L, run->heads, 3 * D, 128};
   const b2_view3 vk{qkv + k0 * 3 * D + D, k_rows, run->heads, 3 * D, 128}, vv{qkv + k0 * 3 * D + 2 * D, k_rows, run->heads, 3 * D, 128};
   const b2_view3 vo{attn, L, run->heads, D, 128};
@@ -217,8 +229,11 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
   b2_attention_options ao = run->attention;
   if (ao.variant == 0) ao.variant = B2_ATTENTION_Q8_FP8_F32ACC;
   const float sm_scale = static_cast<float>(1.0 / std::sqrt(128.0));
-  if (const int rc = b2_attention_q8(&ao, &vq, &vk, &vv, &vo, run->cu_seqlens, cu_k, run->batch, run->max_seqlen, sm_scale,
-                                     base + ws.attn_ws, ws.attn_ws_bytes, st, fused ? &nr : nullptr)) {
+  const b2_qk_norm_rope* norm_rope = fused ? &nr : nullptr;
+  if (const int rc = direct ? attention_rows(&ao, &vq, &vk, &vv, &vo, run->cu_seqlens, cu_k, run->batch, run->max_seqlen, sm_scale,
+                                             base + ws.attn_ws, ws.attn_ws_bytes, st, norm_rope, rows)
+                            : b2_attention_q8(&ao, &vq, &vk, &vv, &vo, run->cu_seqlens, cu_k, run->batch, run->max_seqlen, sm_scale,
+                                              base + ws.attn_ws, ws.attn_ws_bytes, st, norm_rope)) {
     return rc;
   }
 

@@ -797,6 +797,7 @@ int graphed_impl(b2_dit_graphs* g, const b2_dit_model* model, const b2_forward* 
   // What the library sets up once per device and cannot do inside a capture.
   cublasLtHandle_t handle = nullptr;
   if (const int rc = lt_handle(&handle)) return rc;
+  if (const int rc = prepare_situ_tables(stream)) return rc;
 
   GraphEntry entry;
   entry.hash = hash, entry.key = std::move(key);
@@ -971,6 +972,7 @@ int prefill_impl(const b2_dit_model* model, const b2_prefill* prefill, void* str
   for (int bi = 0; bi < m.num_blocks; ++bi) {
     b2_block_run tap = run;
     tap.kv_tap = static_cast<__nv_bfloat16*>(f.kv_out) + static_cast<std::size_t>(bi) * static_cast<std::size_t>(total) * 2 * static_cast<std::size_t>(D);
+    tap.tap_only = bi + 1 == m.num_blocks;  // nothing reads the last block's tokens
     b2_block_buffers bb{};
     bb.struct_size = sizeof bb;
     bb.x = x, bb.mod = mod, bb.rope = rope, bb.workspace = base + c.block, bb.workspace_bytes = c.total - c.block;

@@ -979,6 +979,11 @@ GemmParams base_params(const b2_int8_operands* a) {
 
 }  // namespace
 
+int prepare_situ_tables(cudaStream_t stream) {
+  SituTables t;
+  return situ_tables(stream, &t);
+}
+
 // Used by the block driver (same translation-unit-independent entry points as the C ABI).
 int gemm_status_word(int* host_value) {
   const cudaError_t e = cudaMemcpyFromSymbol(host_value, g_gemm_status, sizeof(int));
