@@ -22,6 +22,24 @@ int fail_cuda(const char* op, cudaError_t e) {
   return fail_status(B2_ERR_CUDA, op, std::string("CUDA error: ") + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")");
 }
 
+namespace {
+struct Chain {
+  cudaStream_t stream = nullptr;
+  bool open = false;
+  int launches = 0;
+};
+thread_local Chain g_chain;
+}  // namespace
+
+LaunchChain::LaunchChain(cudaStream_t stream) : outer_(!g_chain.open) {
+  if (outer_) g_chain = Chain{stream, true, 0};
+}
+LaunchChain::~LaunchChain() {
+  if (outer_) g_chain = Chain{};
+}
+bool in_chain(cudaStream_t stream) { return g_chain.open && g_chain.stream == stream; }
+bool chain_follows(cudaStream_t stream) { return in_chain(stream) && g_chain.launches++ > 0; }
+
 int sm_count() {
   static std::atomic<int> cached[64] = {};
   int dev = 0;

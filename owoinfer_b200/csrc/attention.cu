@@ -180,6 +180,8 @@ struct NormRopeArgs {
 // One warp per (token, q-or-k head), lane l holding channels 4l..4l+3: the quad sum then the shuffle-down tree are the
 // order of torch's reduce for a 128-wide row. RoPE pairs channel d with d + 64, i.e. lane l with lane l ^ 16.
 __global__ void __launch_bounds__(256) qk_norm_rope_kernel(const NormRopeArgs a) {
+  dependents_may_start();
+  wait_for_predecessors();
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const std::int64_t items = a.tokens * 2 * a.heads;
   const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -225,6 +227,8 @@ constexpr RopeBands kBands = {{1.f, 0.562341332f, 0.316227764f, 0.177827939f, 0.
 // Reference tokens of the edit layout (image_r, image_f = reference index + 1, 0; no text rows) use the same arithmetic.
 __global__ void rope_table_kernel(__nv_bfloat16* out, std::int64_t ld, std::int64_t n, int height, int width,
                                   float image_r, float image_f, const RopeBands bands) {
+  dependents_may_start();
+  wait_for_predecessors();
   const std::int64_t hw = static_cast<std::int64_t>(height) * width;
   const float h_mid = static_cast<float>((height - 1) / 2.0), w_mid = static_cast<float>((width - 1) / 2.0);
   const std::int64_t total = n * 128;
@@ -345,6 +349,8 @@ __device__ __forceinline__ void norm_rope_row(const std::uint32_t (&x)[4], const
 // of q and k; Q quantised with the block's scale; k written back in place for the statistics and K/V quantisation
 // passes. Every load of a row is issued before the first use.
 __global__ void __launch_bounds__(512, 2) norm_rope_quant_q_kernel(const PrepArgs p) {
+  dependents_may_start();
+  wait_for_predecessors();
   const int bx = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int lane = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
   const int start = p.cu[b], len = p.cu[b + 1] - start;
@@ -406,6 +412,8 @@ __global__ void __launch_bounds__(512, 2) norm_rope_quant_q_kernel(const PrepArg
 // tokens row, row + 16, ... of the chunk in order; the 16 partials are then added in order, and the finalize kernel adds
 // the chunks in order: the K mean is reproducible and independent of the launch shape. Loads run four tokens ahead.
 __global__ void __launch_bounds__(256) stats_kernel(const PrepArgs p) {
+  dependents_may_start();
+  wait_for_predecessors();
   const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int lane = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
   const int start = p.cu[b], len = p.cu[b + 1] - start;
@@ -464,6 +472,8 @@ __global__ void __launch_bounds__(256) stats_kernel(const PrepArgs p) {
 }
 
 __global__ void __launch_bounds__(kHeadDim) finalize_kernel(const PrepArgs p) {
+  dependents_may_start();
+  wait_for_predecessors();
   const int h = blockIdx.x, b = blockIdx.y, ch = threadIdx.x;
   const int len = p.cu[b + 1] - p.cu[b];
   const std::int64_t base = (static_cast<std::int64_t>(b) * p.heads + h) * p.chunks * kHeadDim + ch;
@@ -480,6 +490,8 @@ __global__ void __launch_bounds__(kHeadDim) finalize_kernel(const PrepArgs p) {
 
 // Q per (32 tokens, head): amax floored at 1e-7, scale = amax / 127, q = rni(x * (127 / amax)). CTA = 32 rows x 16 lanes.
 __global__ void __launch_bounds__(512) quant_q_kernel(const PrepArgs p) {
+  dependents_may_start();
+  wait_for_predecessors();
   const int bx = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int lane = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
   const int start = p.cu[b], len = p.cu[b + 1] - start;
@@ -509,6 +521,8 @@ __global__ void __launch_bounds__(512) quant_q_kernel(const PrepArgs p) {
 // K and V of one (64 keys, head): K - mean -> int8 with one scale; V * v_recp -> e4m3. CTA = 16 rows x 16 lanes, each
 // thread taking keys row, row + 16, row + 32, row + 48 (eight loads in flight per thread, one block-wide maximum).
 __global__ void __launch_bounds__(256) quant_kv_kernel(const PrepArgs p) {
+  dependents_may_start();
+  wait_for_predecessors();
   const int bx = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int lane = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
   const int start = p.cu[b], len = p.cu[b + 1] - start;
@@ -735,6 +749,7 @@ struct AttnArgs {
   int heads, q_blocks, k_blocks;
   float scale_log2;  // sm_scale * log2(e)
   float p_offset;
+  int hand_over;  // let the next kernel start before this one has finished (see kHandOverRows)
   // Test hook (kDump instantiation only): the raw integer scores of one (sequence, head, query tile).
   std::int32_t* dump;
   std::int64_t dump_ld;
@@ -780,6 +795,7 @@ template <bool kDump>
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const AttnArgs a) {
+  wait_for_predecessors();
   const int bq = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int q_start = a.cu_q[b], qo_len = a.cu_q[b + 1] - q_start;
   const int k_start = a.cu_k[b], kv_len = a.cu_k[b + 1] - k_start;
@@ -854,6 +870,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         mbar_expect_tx(smem_u32(&s_v_full[s]), kTileBytes);
         tma_load_2d(v_smem(s), &map_v, smem_u32(&s_v_full[s]), h * kHeadDim, k_start + t * kTileK);
       }
+      if (a.hand_over != 0) dependents_may_start();
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -1240,8 +1257,7 @@ int b2_qk_norm_rope_moss(void* qkv, int64_t ld, int64_t tokens, int heads, const
                        tokens, heads, static_cast<float>(rows) / static_cast<float>(rows * kHeadDim)};
   const std::int64_t items = tokens * 2 * heads;
   const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((items + 7) / 8, 148 * 64));
-  qk_norm_rope_kernel<<<blocks, 256, 0, as_stream(stream)>>>(a);
-  return check_launch(op);
+  return enqueue(op, qk_norm_rope_kernel, blocks, 256, 0, as_stream(stream), 1, a);
 }
 
 int b2_moss_rope_table(void* out, int64_t ld, int height, int width, int text_length, void* stream) {
@@ -1251,9 +1267,8 @@ int b2_moss_rope_table(void* out, int64_t ld, int height, int width, int text_le
   if (n == 0) return B2_OK;
   if (out == nullptr) return fail_invalid(op, "null table");
   const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((n * 128 + 255) / 256, 148 * 32));
-  rope_table_kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<__nv_bfloat16*>(out), ld, n, height, width, 0.f,
-                                                           static_cast<float>(text_length), kBands);
-  return check_launch(op);
+  return enqueue(op, rope_table_kernel, blocks, 256, 0, as_stream(stream), 1, static_cast<__nv_bfloat16*>(out), ld, n, height, width,
+                 0.f, static_cast<float>(text_length), kBands);
 }
 
 int b2_moss_rope_table_reference(void* out, int64_t ld, int height, int width, int index, void* stream) {
@@ -1264,9 +1279,8 @@ int b2_moss_rope_table_reference(void* out, int64_t ld, int height, int width, i
   if (out == nullptr) return fail_invalid(op, "null table");
   const std::int64_t n = static_cast<std::int64_t>(height) * width;
   const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((n * 128 + 255) / 256, 148 * 32));
-  rope_table_kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<__nv_bfloat16*>(out), ld, n, height, width,
-                                                           static_cast<float>(index + 1), 0.f, kBands);
-  return check_launch(op);
+  return enqueue(op, rope_table_kernel, blocks, 256, 0, as_stream(stream), 1, static_cast<__nv_bfloat16*>(out), ld, n, height, width,
+                 static_cast<float>(index + 1), 0.f, kBands);
 }
 
 size_t b2_attention_q8_workspace_bytes(const b2_attention_options* o, int64_t total_q, int64_t total_k, int batch,
@@ -1342,6 +1356,7 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     return fail_invalid(op, "workspace too small or not 256-byte aligned (need " + std::to_string(l.total) + " bytes)");
   }
   cudaStream_t st = as_stream(stream);
+  const LaunchChain chain(st);
   auto* base = static_cast<std::uint8_t*>(workspace);
   PrepArgs p{};
   p.q = static_cast<const __nv_bfloat16*>(q->data), p.k = static_cast<__nv_bfloat16*>(k->data);
@@ -1378,21 +1393,16 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     p.norm_factor = static_cast<float>(norm_rows) / static_cast<float>(norm_rows * kHeadDim);
     PrepArgs own = p;  // queries and the key rows of the same tokens
     own.cu = cu_seqlens_q, own.k = p.k + p.own0 * p.k_row;
-    norm_rope_quant_q_kernel<<<dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st>>>(own);
-    if (const int rc = check_launch(op)) return rc;
+    if (const int rc = enqueue(op, norm_rope_quant_q_kernel, dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st, 1, own)) return rc;
   }
-  stats_kernel<<<stats_grid, 256, 0, st>>>(p);
-  if (const int rc = check_launch(op)) return rc;
-  finalize_kernel<<<dim3(static_cast<unsigned>(heads), batch), kHeadDim, 0, st>>>(p);
-  if (const int rc = check_launch(op)) return rc;
+  if (const int rc = enqueue(op, stats_kernel, stats_grid, 256, 0, st, 1, p)) return rc;
+  if (const int rc = enqueue(op, finalize_kernel, dim3(static_cast<unsigned>(heads), batch), kHeadDim, 0, st, 1, p)) return rc;
   if (norm_rope == nullptr) {
     PrepArgs pq = p;
     pq.cu = cu_seqlens_q;
-    quant_q_kernel<<<dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st>>>(pq);
-    if (const int rc = check_launch(op)) return rc;
+    if (const int rc = enqueue(op, quant_q_kernel, dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st, 1, pq)) return rc;
   }
-  quant_kv_kernel<<<dim3(l.k_blocks, static_cast<unsigned>(heads), batch), 256, 0, st>>>(p);
-  if (const int rc = check_launch(op)) return rc;
+  if (const int rc = enqueue(op, quant_kv_kernel, dim3(l.k_blocks, static_cast<unsigned>(heads), batch), 256, 0, st, 1, p)) return rc;
   if (prepass_only) return B2_OK;
 
   CUtensorMap map_q, map_k, map_v;
@@ -1409,6 +1419,7 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   a.heads = static_cast<int>(heads), a.q_blocks = l.q_blocks, a.k_blocks = l.k_blocks;
   a.scale_log2 = scale * 1.44269504088896340736f;
   a.p_offset = p_offset_of(p_range);
+  a.hand_over = total_q <= kHandOverRows;
   if (dump != nullptr) {
     a.dump = dump->scores, a.dump_ld = dump->ld;
     a.dump_seq = dump->seq, a.dump_head = dump->head, a.dump_tile = dump->tile;
@@ -1426,8 +1437,7 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     return fail_cuda(op, e);
   }
   const dim3 grid((max_seqlen + kTileQ - 1) / kTileQ, static_cast<unsigned>(heads), batch);
-  kernel<<<grid, kAttnThreads, kAttnSmem, st>>>(map_q, map_k, map_v, a);
-  return check_launch(op);
+  return enqueue(op, kernel, grid, kAttnThreads, kAttnSmem, st, 1, map_q, map_k, map_v, a);
 }
 }  // namespace
 }  // extern "C"

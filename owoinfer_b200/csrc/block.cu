@@ -133,6 +133,7 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
   const std::int64_t L = run->tokens, D = run->D, F = run->F;
   if (L == 0) return B2_OK;
   cudaStream_t st = as_stream(stream);
+  const LaunchChain chain(st);
   auto* base = static_cast<std::uint8_t*>(a->workspace);
   auto* xq = reinterpret_cast<std::int8_t*>(base + ws.xq);
   auto* scale = reinterpret_cast<float*>(base + ws.scale);
@@ -166,6 +167,7 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
     const float* wsc = nullptr;
     if (const int rc = site_operands(op, lin, run->tier, w_unpack, n, k, st, &wq, &wsc)) return rc;
     const b2_int8_operands o{xq, k, scale, wq, wsc, L, n, k};
+    if (run->tier == B2_TIER_INT8) return gemm_site(&o, epilogue, aux, out, ldo, st);
     if (epilogue == 0) return b2_int8_gemm(&o, aux, out, ldo, st, B2_TILE_AUTO);
     if (epilogue == 1) return b2_int8_gemm_gated_residual(&o, nullptr, aux, out, ldo, st, B2_TILE_AUTO);
     return b2_int8_gemm_situ_glu(&o, out, ldo, st, B2_TILE_AUTO);
@@ -271,6 +273,7 @@ int b2_debug_bounded_wait(uint64_t wait_limit_ns, int skip_gemm_stage) {
 int b2_dit_step(const b2_block_weights* blocks, int num_blocks, const b2_block_buffers* a, const b2_block_run* run,
                 void* stream) {
   if (blocks == nullptr || num_blocks < 0) return fail_invalid("dit_step", "null blocks");
+  const LaunchChain chain(as_stream(stream));
   for (int i = 0; i < num_blocks; ++i) {
     if (const int rc = b2_run_block_quant(&blocks[i], a, run, stream)) return rc;
   }

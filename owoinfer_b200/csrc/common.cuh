@@ -36,6 +36,65 @@ int attn_status_clear();
 // Test hooks of the GEMM kernel's bounded waits: the limit in nanoseconds (0 = leave it) and the "skip one stage" switch.
 int gemm_debug_set(unsigned long long wait_limit_ns, int skip_stage);
 
+// ---------------------------------------------------------------------------------------------------------------
+// Host: launches that overlap their predecessor's tail (programmatic dependent launch). While a LaunchChain is alive on
+// this thread, every kernel that enqueue() puts on its stream after the chain's first one may become resident as soon as
+// all blocks of the kernel before it have started; the kernels call dependents_may_start() first thing and
+// wait_for_predecessors() before they touch memory that anything on the stream may still be writing or reading. The
+// chain's first launch is an ordinary one, so whatever a caller enqueued before a call of this library is finished before
+// the call's first kernel starts: data that no kernel of the call writes may be read ahead of the wait.
+// At 2 x 320 tokens a launch takes the GPU about 2 us from the end of one kernel to the first instructions of the next
+// and another 1 to 2 us of set-up, thirteen times per block.
+// ---------------------------------------------------------------------------------------------------------------
+class LaunchChain {
+ public:
+  explicit LaunchChain(cudaStream_t stream);
+  ~LaunchChain();
+  LaunchChain(const LaunchChain&) = delete;
+  LaunchChain& operator=(const LaunchChain&) = delete;
+
+ private:
+  bool outer_;  // this object opened the chain (inner ones on the same stream join it)
+};
+// Whether the launch about to be made on `stream` may overlap its predecessor; counts it as made.
+bool chain_follows(cudaStream_t stream);
+// Inside a chain on `stream`: memory that was complete before the call is constant for all of it.
+bool in_chain(cudaStream_t stream);
+
+template <typename... Params, typename... Args>
+int enqueue(const char* op, void (*kernel)(Params...), dim3 grid, dim3 block, std::size_t smem, cudaStream_t stream, int cluster,
+            const Args&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+  cudaLaunchAttribute attr[2]{};
+  unsigned n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = static_cast<unsigned>(cluster), attr[n].val.clusterDim.y = 1, attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (chain_follows(stream)) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr, cfg.numAttrs = n;
+  if (const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...); e != cudaSuccess) {
+    cudaGetLastError();
+    return fail_cuda(op, e);
+  }
+  return B2_OK;
+}
+
+// Rows up to which the tensor-core kernels, too, let their successor start early (the memory-bound ones always do): 2.5 % of
+// a step at 297 rows, nothing at 647, and from a few thousand rows on it costs 1 % (the early blocks of the next kernel
+// fill up the first SMs to finish).
+constexpr std::int64_t kHandOverRows = 512;
+
+// An INT8 linear of a block run (epilogue 0 plain, 1 gated residual with gate `aux`, 2 SiTU-GLU) whose weight no kernel of
+// the running chain writes: its first tiles are fetched ahead of the wait for the kernel that makes the activations.
+int gemm_site(const b2_int8_operands* o, int epilogue, const void* aux, void* out, std::int64_t ldo, void* stream);
+
 // Fills the SiTU factor tables of the current device once (on `stream`, which it synchronises the first time); a no-op
 // afterwards. For callers that are about to capture: inside a capture every SiTU-GLU launch would bring a fill along.
 int prepare_situ_tables(cudaStream_t stream);
@@ -94,6 +153,10 @@ __device__ __forceinline__ std::uint32_t float_to_bf_bits(float v) {
 __device__ __forceinline__ std::uint32_t smem_u32(const void* p) {
   return static_cast<std::uint32_t>(__cvta_generic_to_shared(p));
 }
+
+// Programmatic dependent launch (see LaunchChain): both are no-ops in a kernel launched the ordinary way.
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_init(std::uint32_t bar, std::uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

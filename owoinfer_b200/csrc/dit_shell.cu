@@ -37,6 +37,8 @@ struct ParamWords {
   std::uint32_t words[kParamWords];
 };
 __global__ void write_words_kernel(std::uint32_t* dst, const ParamWords p, int n) {
+  dependents_may_start();
+  wait_for_predecessors();
   for (int i = static_cast<int>(threadIdx.x); i < n; i += static_cast<int>(blockDim.x)) dst[i] = p.words[i];
 }
 int write_words(const char* op, void* dst, const void* src, std::size_t words, cudaStream_t stream) {
@@ -45,8 +47,7 @@ int write_words(const char* op, void* dst, const void* src, std::size_t words, c
     const int n = static_cast<int>(std::min<std::size_t>(kParamWords, words - at));
     ParamWords p;
     std::memcpy(p.words, from + at, static_cast<std::size_t>(n) * 4);
-    write_words_kernel<<<1, 256, 0, stream>>>(static_cast<std::uint32_t*>(dst) + at, p, n);
-    if (const int rc = check_launch(op)) return rc;
+    if (const int rc = enqueue(op, write_words_kernel, 1, 256, 0, stream, 1, static_cast<std::uint32_t*>(dst) + at, p, n)) return rc;
   }
   return B2_OK;
 }
@@ -54,6 +55,8 @@ int write_words(const char* op, void* dst, const void* src, std::size_t words, c
 // kernels::silu (src/kernels/basic/elementwise.cu:92-100, detail.h:100): bf16(x / (1 + expf(-x))), the division and the
 // addition each rounded once.
 __global__ void silu_bf16_kernel(const __nv_bfloat16* x, __nv_bfloat16* out, std::int64_t n) {
+  dependents_may_start();
+  wait_for_predecessors();
   for (std::int64_t i = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
     const float v = __bfloat162float(x[i]);
@@ -65,6 +68,8 @@ __global__ void silu_bf16_kernel(const __nv_bfloat16* x, __nv_bfloat16* out, std
 // f32 -> bf16 (round to nearest even) or bf16 -> f32.
 template <typename In, typename Out>
 __global__ void __launch_bounds__(kTile * 8) transpose_kernel(const In* in, Out* out, std::int64_t rows, std::int64_t cols, std::int64_t ld) {
+  dependents_may_start();
+  wait_for_predecessors();
   __shared__ float tile[kTile][kTile + 1];
   const std::int64_t r0 = static_cast<std::int64_t>(blockIdx.y) * kTile, c0 = static_cast<std::int64_t>(blockIdx.x) * kTile;
   const int tx = static_cast<int>(threadIdx.x);
@@ -89,8 +94,7 @@ template <typename In, typename Out>
 int launch_transpose(const char* op, const In* in, Out* out, std::int64_t rows, std::int64_t cols, std::int64_t ld, cudaStream_t stream) {
   if (rows == 0 || cols == 0) return B2_OK;
   const dim3 grid(static_cast<unsigned>((cols + kTile - 1) / kTile), static_cast<unsigned>((rows + kTile - 1) / kTile));
-  transpose_kernel<In, Out><<<grid, dim3(kTile, 8), 0, stream>>>(in, out, rows, cols, ld);
-  return check_launch(op);
+  return enqueue(op, transpose_kernel<In, Out>, grid, dim3(kTile, 8), 0, stream, 1, in, out, rows, cols, ld);
 }
 
 // One warp per output row, 8 weights per 16-byte load: lane l takes chunks l, l + 32, ... and accumulates with one fma
@@ -98,6 +102,8 @@ int launch_transpose(const char* op, const In* in, Out* out, std::int64_t rows, 
 // out = bf16(sum + bias). The order of every operation is the reference kernel's, so the bits are.
 __global__ void __launch_bounds__(256) linear_fp32_row_kernel(const __nv_bfloat16* w, const float* x, const float* bias,
                                                               __nv_bfloat16* out, int n, int k) {
+  dependents_may_start();
+  wait_for_predecessors();
   const int row = static_cast<int>(blockIdx.x) * (static_cast<int>(blockDim.x) / 32) + static_cast<int>(threadIdx.x) / 32;
   const int lane = static_cast<int>(threadIdx.x) % 32;
   if (row >= n) return;
@@ -345,9 +351,8 @@ int b2_linear_fp32_row(const void* w, const float* x, const float* bias, void* o
   if (w == nullptr || x == nullptr || bias == nullptr || out == nullptr || !aligned_to(w, 16) || !aligned_to(x, 16)) {
     return fail_invalid(op, "needs a 16-byte aligned bf16 w [n, k], a 16-byte aligned f32 x [k], an f32 bias [n] and a bf16 out [n]");
   }
-  linear_fp32_row_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, as_stream(stream)>>>(
-      static_cast<const __nv_bfloat16*>(w), x, bias, static_cast<__nv_bfloat16*>(out), n, k);
-  return check_launch(op);
+  return enqueue(op, linear_fp32_row_kernel, static_cast<unsigned>((n + 7) / 8), 256, 0, as_stream(stream), 1,
+                 static_cast<const __nv_bfloat16*>(w), x, bias, static_cast<__nv_bfloat16*>(out), n, k);
 }
 
 int b2_time_sinusoid(float timestep, float* emb) {
@@ -405,8 +410,7 @@ int b2_silu_bf16(const void* x, void* out, int64_t n, void* stream) {
   if (n < 0 || (n > 0 && (x == nullptr || out == nullptr))) return fail_invalid(op, "needs bf16 x and out of n values");
   if (n == 0) return B2_OK;
   const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((n + 255) / 256, 4096));
-  silu_bf16_kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), n);
-  return check_launch(op);
+  return enqueue(op, silu_bf16_kernel, blocks, 256, 0, as_stream(stream), 1, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), n);
 }
 
 size_t b2_time_modulation_bf16_workspace_bytes(const b2_time_mlp_bf16* m) {
@@ -546,6 +550,7 @@ int dit_forward_impl(const b2_dit_model* model, const b2_forward* forward, const
     return fail_invalid(op, "workspace must be 256-byte aligned and hold b2_dit_forward_workspace_bytes() = " + std::to_string(c.total));
   }
   cudaStream_t stream = as_stream(stream_);
+  const LaunchChain chain(stream);
   const std::int64_t hw = static_cast<std::int64_t>(f.height) * f.width, D = m.D;
   unsigned char* base = static_cast<unsigned char*>(f.workspace);
   __nv_bfloat16* x = reinterpret_cast<__nv_bfloat16*>(base + c.x);
@@ -949,6 +954,7 @@ int prefill_impl(const b2_dit_model* model, const b2_prefill* prefill, void* str
     return fail_invalid(op, "workspace must be 256-byte aligned and hold b2_dit_prefill_workspace_bytes() = " + std::to_string(c.total));
   }
   cudaStream_t stream = as_stream(stream_);
+  const LaunchChain chain(stream);
   const std::int64_t D = m.D;
   unsigned char* base = static_cast<unsigned char*>(f.workspace);
   __nv_bfloat16* x = reinterpret_cast<__nv_bfloat16*>(base + c.x);

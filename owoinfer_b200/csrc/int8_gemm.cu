@@ -91,6 +91,10 @@ struct GemmParams {
   int w4_group_shift;  // log2(group)
   const float* w4_codebook;
   unsigned* w4_invalid;
+  // Reads that need not wait for the kernels before this one: the weight (no kernel of the call writes it) and the SiTU
+  // tables (filled long ago).
+  int early_weight, early_tables;
+  int hand_over;  // let the next kernel start before this one has finished (see kHandOverRows)
 };
 
 __device__ int g_gemm_status = 0;  // set to 1 by a CTA whose bounded wait expired
@@ -269,6 +273,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   }
   if constexpr (kEpi == Epi::kSituGlu) {
+    if (p.early_tables == 0) wait_for_predecessors();
     for (int i = threadIdx.x; i < kMiniGate + kMiniHidden; i += blockDim.x) {
       const bool gate = i < kMiniGate;
       const std::uint32_t j = gate ? i : i - kMiniGate;  // [sign (gate only)][exponent][mantissa]
@@ -289,11 +294,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   if (warp == 0) {
     if (lane == 0) {
       std::uint32_t it = 0;
-      for (int tile = tile0; tile < total_tiles && *abort_word == 0; tile += tile_step) {
-        int mt, nt;
-        tile_coords(p, tile, &mt, &nt);
-        const int row_a = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM;
-        int row_b0, row_b1;
+      // First rows of this CTA's two 128-row parts of a B tile (a pair's CTA has one: its own half).
+      const auto b_rows = [&](int nt, int& row_b0, int& row_b1) {
         if constexpr (kEpi == Epi::kSituGlu) {
           row_b0 = nt * 128;
           row_b1 = p.half + nt * 128;
@@ -302,6 +304,36 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           row_b1 = nt * kBN + 128;
         }
         if (kCtas == 2 && rank == 1) row_b0 = row_b1;  // the pair's second CTA stages the second 128 rows of B
+      };
+      // The first stages' weight tiles, ahead of the wait: they come from HBM, the activations were just written.
+      std::uint32_t ahead = 0;
+      if constexpr (!kW4) {
+        if (p.early_weight != 0 && tile0 < total_tiles && g_gemm_test_skip_stage == 0) {
+          int mt, nt, row_b0, row_b1;
+          tile_coords(p, tile0, &mt, &nt);
+          b_rows(nt, row_b0, row_b1);
+          ahead = static_cast<std::uint32_t>(min(kStages, k_blocks));
+          for (std::uint32_t s = 0; s < ahead; ++s) {
+            const std::uint32_t full = smem_u32(&s_full[s]);
+            const int c0 = static_cast<int>(s) * kBK;
+            if constexpr (kCtas == 2) {
+              if (rank == 0) mbar_expect_tx(full, 2 * S::kStageBytes);
+              tma_load_2d_pair(b_addr(s), &map_b, map_to_cta(full, 0), c0, row_b0);
+            } else {
+              mbar_expect_tx(full, S::kStageBytes);
+              tma_load_2d(b_addr(s), &map_b, full, c0, row_b0);
+              if constexpr (kBN == 256) tma_load_2d(b_addr(s) + 128 * kBK, &map_b, full, c0, row_b1);
+            }
+          }
+        }
+      }
+      wait_for_predecessors();
+      for (int tile = tile0; tile < total_tiles && *abort_word == 0; tile += tile_step) {
+        int mt, nt;
+        tile_coords(p, tile, &mt, &nt);
+        const int row_a = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM;
+        int row_b0, row_b1;
+        b_rows(nt, row_b0, row_b1);
         const bool skip_last = g_gemm_test_skip_stage != 0 && tile == tile0;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = static_cast<int>(it % kStages);
@@ -322,6 +354,9 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const std::uint32_t pfull = smem_u32(&s_pfull[s]);
             mbar_expect_tx(pfull, S::kPBytes);
             tma_load_2d(p_addr(s), &map_b, pfull, kb * (kBK / 2), row_b0);
+          } else if (it < ahead) {  // the weight tile is on its way already
+            if constexpr (kCtas == 2) tma_load_2d_pair(a_addr(s), &map_a, map_to_cta(full, 0), kb * kBK, row_a);
+            else tma_load_2d(a_addr(s), &map_a, full, kb * kBK, row_a);
           } else if constexpr (kCtas == 2) {
             // Both CTAs' copies complete on the leader's barrier, which expects the bytes of the whole pair.
             if (rank == 0) mbar_expect_tx(full, 2 * S::kStageBytes);
@@ -336,6 +371,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           }
         }
       }
+      // Every load is on its way: what follows may set itself up under the last tile's epilogue.
+      if (p.hand_over != 0) dependents_may_start();
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -394,6 +431,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // K block ahead) and writes the 64 INT8 values into the B stage in the 128-byte-swizzled layout the MMA reads (chunk
     // n of row r at n ^ (r % 8)); then the warp arrives on the stage's "full" barrier (the leader's, for a pair) in place
     // of a TMA completion.
+    wait_for_predecessors();
     const int ct = (warp - 2 - kEpiWarps) * 32 + lane;
     const int r = ct & 127, half = ct >> 7;
     const int groups = p.k >> p.w4_group_shift;
@@ -476,6 +514,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // Epilogue: 8 warps. Warp w may touch TMEM lanes [32 (w % 4), 32 (w % 4) + 32); warps 2..5 take the first half of the
     // tile's columns, warps 6..9 the second half (SiTU-GLU: output columns, each needing its hidden and gate accumulator).
     const int quarter = warp & 3, col_half = (warp - 2) >> 2;  // SiTU-GLU: one of four 32-column parts
+    wait_for_predecessors();
     std::uint32_t tile_it = 0;
     for (int tile = tile0; tile < total_tiles; tile += tile_step, ++tile_it) {
       int mt, nt;
@@ -762,6 +801,7 @@ __global__ void fill_situ_tables() {
 struct SituTables {
   const std::uint16_t* gate = nullptr;
   const std::uint16_t* hidden = nullptr;
+  bool ready = false;  // filled by an earlier call (not by a kernel this call puts on the stream)
 };
 
 // Filled once per device. Outside stream capture the first call fills on `stream` and synchronises it (the one host
@@ -782,6 +822,7 @@ int situ_tables(cudaStream_t stream, SituTables* out) {
     ptrs[dev].gate = static_cast<const std::uint16_t*>(g);
     ptrs[dev].hidden = static_cast<const std::uint16_t*>(h);
   }
+  out->ready = filled[dev];
   if (!filled[dev]) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (const cudaError_t e = cudaStreamIsCapturing(stream, &cap); e != cudaSuccess) return fail_cuda(op, e);
@@ -792,7 +833,7 @@ int situ_tables(cudaStream_t stream, SituTables* out) {
       filled[dev] = true;
     }
   }
-  *out = ptrs[dev];
+  out->gate = ptrs[dev].gate, out->hidden = ptrs[dev].hidden;
   return B2_OK;
 }
 
@@ -902,23 +943,8 @@ int launch_kernel(const char* op, const b2_int8_operands* a, GemmParams p, cudaS
       p.band_m = std::max(p.band_m, static_cast<int>(resident));
     }
   }
-  if constexpr (kCtas == 2) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * std::min(total, sm_count() / 2)));
-    cfg.blockDim = dim3(threads_of(kEpi, kBN, kW4));
-    cfg.dynamicSmemBytes = S::kSmemBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr, cfg.numAttrs = 1;
-    if (const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, p); e != cudaSuccess) return fail_cuda(op, e);
-    return check_launch(op);
-  } else {
-    const int grid = std::min(total, sm_count());
-    kernel<<<grid, threads_of(kEpi, kBN, kW4), S::kSmemBytes, stream>>>(map_a, map_b, p);
-    return check_launch(op);
-  }
+  const int grid = kCtas == 2 ? 2 * std::min(total, sm_count() / 2) : std::min(total, sm_count());
+  return enqueue(op, kernel, grid, threads_of(kEpi, kBN, kW4), S::kSmemBytes, stream, kCtas, map_a, map_b, p);
 }
 
 // Tile choice: CTA pairs on 256 x 256 tiles when there are enough of them to fill the GPU; else one CTA per 128 x 256
@@ -974,6 +1000,7 @@ GemmParams base_params(const b2_int8_operands* a) {
   GemmParams p{};
   p.m = static_cast<int>(a->m), p.n = static_cast<int>(a->n), p.k = static_cast<int>(a->k);
   p.xs = a->x_scale, p.ws = a->w_scale;
+  p.hand_over = a->m <= kHandOverRows;
   return p;
 }
 
@@ -1042,14 +1069,74 @@ int check_situ(const char* op, const b2_int8_operands* a, const void* out, std::
 
 extern "C" {
 
-int b2_int8_gemm(const b2_int8_operands* op_, const void* bias, void* out, int64_t ldo, void* stream, int tile) {
+}  // extern "C"
+
+namespace b2 {
+namespace {
+
+int gemm_plain(const b2_int8_operands* op_, const void* bias, void* out, int64_t ldo, void* stream, int tile, bool early_weight) {
   constexpr const char* op = "int8_gemm";
   if (const int rc = check_plain(op, op_, bias, out, ldo)) return rc;
   if (op_->m == 0) return B2_OK;
   GemmParams p = base_params(op_);
+  p.early_weight = early_weight;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.out = static_cast<__nv_bfloat16*>(out), p.ldo = ldo;
   return dispatch<Epi::kPlain>(op, op_, p, as_stream(stream), tile);
+}
+
+int gemm_gated(const b2_int8_operands* op_, const void* bias, const void* gate, void* residual, int64_t ldr, void* stream, int tile,
+               bool early_weight) {
+  constexpr const char* op = "int8_gemm_gated_residual";
+  if (const int rc = check_gated(op, op_, bias, gate, residual, ldr)) return rc;
+  if (op_->m == 0) return B2_OK;
+  GemmParams p = base_params(op_);
+  p.early_weight = early_weight;
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.gate = static_cast<const __nv_bfloat16*>(gate);
+  p.out = static_cast<__nv_bfloat16*>(residual), p.ldo = ldr;
+  return dispatch<Epi::kGatedResidual>(op, op_, p, as_stream(stream), tile);
+}
+
+int gemm_situ(const b2_int8_operands* op_, void* out, int64_t ldo, void* stream, int tile, bool early_weight) {
+  constexpr const char* op = "int8_gemm_situ_glu";
+  if (const int rc = check_situ(op, op_, out, ldo)) return rc;
+  if (op_->m == 0) return B2_OK;
+  SituTables t;
+  if (const int rc = situ_tables(as_stream(stream), &t)) return rc;
+  GemmParams p = base_params(op_);
+  p.early_weight = early_weight;
+  p.half = static_cast<int>(op_->n / 2);
+  p.out = static_cast<__nv_bfloat16*>(out), p.ldo = ldo;
+  p.situ_wide = aligned_to(out, 16) && ldo % 8 == 0 && p.half % 8 == 0;
+  p.t_gate = t.gate, p.t_hidden = t.hidden, p.early_tables = t.ready;
+  return dispatch<Epi::kSituGlu>(op, op_, p, as_stream(stream), tile);
+}
+
+}  // namespace
+
+int gemm_site(const b2_int8_operands* o, int epilogue, const void* aux, void* out, std::int64_t ldo, void* stream) {
+  const bool early = in_chain(as_stream(stream));
+  if (epilogue == 0) return gemm_plain(o, aux, out, ldo, stream, B2_TILE_AUTO, early);
+  if (epilogue == 1) return gemm_gated(o, nullptr, aux, out, ldo, stream, B2_TILE_AUTO, early);
+  return gemm_situ(o, out, ldo, stream, B2_TILE_AUTO, early);
+}
+
+}  // namespace b2
+
+extern "C" {
+
+int b2_int8_gemm(const b2_int8_operands* op, const void* bias, void* out, int64_t ldo, void* stream, int tile) {
+  return gemm_plain(op, bias, out, ldo, stream, tile, false);
+}
+
+int b2_int8_gemm_gated_residual(const b2_int8_operands* op, const void* bias, const void* gate, void* residual, int64_t ldr,
+                                void* stream, int tile) {
+  return gemm_gated(op, bias, gate, residual, ldr, stream, tile, false);
+}
+
+int b2_int8_gemm_situ_glu(const b2_int8_operands* op, void* out, int64_t ldo, void* stream, int tile) {
+  return gemm_situ(op, out, ldo, stream, tile, false);
 }
 
 int b2_int8_gemm_chunked(const b2_int8_operands* op_, const void* bias, void* out, int64_t ldo, int chunk_cols,
@@ -1067,32 +1154,6 @@ int b2_int8_gemm_chunked(const b2_int8_operands* op_, const void* bias, void* ou
   p.out = static_cast<__nv_bfloat16*>(out), p.ldo = ldo;
   p.chunk_cols = chunk_cols, p.chunk_stride = chunk_stride;
   return dispatch<Epi::kPlain>(op, op_, p, as_stream(stream), tile);
-}
-
-int b2_int8_gemm_gated_residual(const b2_int8_operands* op_, const void* bias, const void* gate, void* residual,
-                                int64_t ldr, void* stream, int tile) {
-  constexpr const char* op = "int8_gemm_gated_residual";
-  if (const int rc = check_gated(op, op_, bias, gate, residual, ldr)) return rc;
-  if (op_->m == 0) return B2_OK;
-  GemmParams p = base_params(op_);
-  p.bias = static_cast<const __nv_bfloat16*>(bias);
-  p.gate = static_cast<const __nv_bfloat16*>(gate);
-  p.out = static_cast<__nv_bfloat16*>(residual), p.ldo = ldr;
-  return dispatch<Epi::kGatedResidual>(op, op_, p, as_stream(stream), tile);
-}
-
-int b2_int8_gemm_situ_glu(const b2_int8_operands* op_, void* out, int64_t ldo, void* stream, int tile) {
-  constexpr const char* op = "int8_gemm_situ_glu";
-  if (const int rc = check_situ(op, op_, out, ldo)) return rc;
-  if (op_->m == 0) return B2_OK;
-  SituTables t;
-  if (const int rc = situ_tables(as_stream(stream), &t)) return rc;
-  GemmParams p = base_params(op_);
-  p.half = static_cast<int>(op_->n / 2);
-  p.out = static_cast<__nv_bfloat16*>(out), p.ldo = ldo;
-  p.situ_wide = aligned_to(out, 16) && ldo % 8 == 0 && p.half % 8 == 0;
-  p.t_gate = t.gate, p.t_hidden = t.hidden;
-  return dispatch<Epi::kSituGlu>(op, op_, p, as_stream(stream), tile);
 }
 
 int b2_int8_gemm_acc(const b2_int8_operands* op_, int32_t* acc, int64_t ldacc, void* stream, int tile) {
@@ -1154,7 +1215,7 @@ int b2_w4a8_gemm(const int8_t* x_q, int64_t ldx, const float* x_scale, const b2_
     }
     SituTables t;
     if (const int rc = situ_tables(as_stream(stream), &t)) return rc;
-    p.half = static_cast<int>(n / 2), p.t_gate = t.gate, p.t_hidden = t.hidden;
+    p.half = static_cast<int>(n / 2), p.t_gate = t.gate, p.t_hidden = t.hidden, p.early_tables = t.ready;
     p.situ_wide = aligned_to(out, 16) && ldo % 8 == 0 && p.half % 8 == 0;
     return dispatch_w4<Epi::kSituGlu>(op, &f, p, as_stream(stream));
   }

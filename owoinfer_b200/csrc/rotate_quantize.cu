@@ -182,6 +182,8 @@ constexpr int kNormSmemMaxK = 4096;  // rows up to this length sum their squares
 // scattered into a shared tile in natural order, so each lane stores 16 (INT8) or 8 (INT4) contiguous bytes per group.
 template <int kPairs, bool kNorm, bool kInt4>
 __global__ void __launch_bounds__(kPairs == 1 ? 384 : 512, kPairs == 1 ? 2 : 1) rotate_quantize_kernel(const Args a, const int m) {
+  dependents_may_start();
+  wait_for_predecessors();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ u32 s_warp_max[4][16];
   __shared__ float s_inv_rms;
@@ -533,8 +535,7 @@ int launch_shape(const char* op, const Args& a, std::int64_t m, int threads, std
     slot.store(per_sm, std::memory_order_release);
   }
   const std::int64_t blocks = std::min<std::int64_t>(m, static_cast<std::int64_t>(sm_count()) * per_sm);
-  kernel<<<static_cast<unsigned>(blocks), static_cast<unsigned>(threads), smem, stream>>>(a, static_cast<int>(m));
-  return check_launch(op);
+  return enqueue(op, kernel, static_cast<unsigned>(blocks), static_cast<unsigned>(threads), smem, stream, 1, a, static_cast<int>(m));
 }
 
 template <bool kNorm, bool kInt4>
@@ -587,6 +588,8 @@ constexpr int kUnpackUnroll = 4;
 template <bool kFlat>
 __global__ void __launch_bounds__(256) unpack_int4_kernel(const std::uint8_t* packed, std::int64_t ldp, std::int8_t* out,
                                                           std::int64_t ldo, std::int64_t items, unsigned per_row) {
+  dependents_may_start();
+  wait_for_predecessors();
   const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
   for (std::int64_t i0 = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < items; i0 += kUnpackUnroll * stride) {
     uint2 in[kUnpackUnroll];
@@ -652,6 +655,8 @@ template <bool kTable>
 __global__ void __launch_bounds__(256) decode_grouped_kernel(const std::uint8_t* packed, const void* s_rel, const float* codebook,
                                                              std::int64_t items, int group, int shift, std::int8_t* out,
                                                              unsigned* invalid) {
+  dependents_may_start();
+  wait_for_predecessors();
   __shared__ float s_cb[16];
   __shared__ uint4 s_table[kTable ? 256 : 1];
   if (threadIdx.x < 16) s_cb[threadIdx.x] = codebook != nullptr ? codebook[threadIdx.x] : static_cast<float>(threadIdx.x) - 8.0f;
@@ -860,8 +865,8 @@ int b2_unpack_int4(const void* packed, int64_t ldp, int8_t* out, int64_t ldo, in
   const std::int64_t total = rows * (k / 16);
   const unsigned blocks = static_cast<unsigned>(std::min<std::int64_t>((total + 256 * kUnpackUnroll - 1) / (256 * kUnpackUnroll), sm_count() * 8LL));
   const auto kernel = ldp == k / 2 && ldo == k ? unpack_int4_kernel<true> : unpack_int4_kernel<false>;
-  kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const std::uint8_t*>(packed), ldp, static_cast<std::int8_t*>(out), ldo, total, static_cast<unsigned>(k / 16));
-  return check_launch(op);
+  return enqueue(op, kernel, blocks, 256, 0, as_stream(stream), 1, static_cast<const std::uint8_t*>(packed), ldp, out, ldo, total,
+                 static_cast<unsigned>(k / 16));
 }
 
 int b2_decode_grouped_int8(const void* packed, const void* s_rel, int scale_kind, const float* codebook, int64_t rows,
@@ -889,8 +894,8 @@ int b2_decode_grouped_int8(const void* packed, const void* s_rel, int scale_kind
     }
   }
   const auto kernel = scale_kind == 0 ? decode_grouped_kernel<true> : decode_grouped_kernel<false>;
-  kernel<<<blocks, 256, 0, as_stream(stream)>>>(static_cast<const std::uint8_t*>(packed), s_rel, codebook, total, group, shift, out, invalid);
-  return check_launch(op);
+  return enqueue(op, kernel, blocks, 256, 0, as_stream(stream), 1, static_cast<const std::uint8_t*>(packed), s_rel, codebook, total,
+                 group, shift, out, invalid);
 }
 
 int b2_w4_invalid_scales(unsigned* host_value, int clear) {

@@ -86,3 +86,24 @@ def test_tap_and_slots_read_in_place_equal_the_copied_forms(ops, slot, n0, n1):
     assert np.array_equal(run(slot_kv=(aligned, aligned), fused_norm_rope=0, **both), want)
     one = dict(slot_rows=slot, cu_seqlens_k=synth.cu_seqlens([n0, n1 + slot]), k0=slot, k1=L + 2 * slot, extra=slot)
     assert np.array_equal(run(slot_kv=(None, aligned), **one), run(slot_kv=(None, shifted), **one))
+
+
+@pytest.mark.parametrize("rows", [33, 512, 513])   # the tensor-core kernels let their successor start early up to 512 rows
+def test_overlapping_launches_change_no_bit(ops, rows):
+    """A step of several blocks, whose launches overlap, against its blocks one by one with a synchronisation after each."""
+    F = 512
+    ws = [synth.block_weights(D, F, 50 + i) for i in range(3)]
+    bws = [ops.BlockWeights(w["norm1"], w["norm2"], w["q_norm"], w["k_norm"], w["qkv"], w["o"], w["up_gate"], w["down"]) for w in ws]
+    mod, rope, x0 = synth.modulation(D, 4), ops.moss_rope_table(1, 1, rows - 1), synth.activations(rows, D, 9)
+    run = ops.block_run(rows, synth.cu_seqlens([rows]), rows, D=D, F=F)
+    work = torch.empty(ops.block_quant_workspace_bytes(run), dtype=torch.uint8, device="cuda")
+    one, many = x0.clone(), [x0.clone() for _ in range(4)]
+    torch.cuda.synchronize()
+    for b in bws:
+        ops.run_block_quant(b, ops.block_buffers(one, mod, rope, work), run)
+        torch.cuda.synchronize()
+    for x in many:
+        ops.dit_step(bws, ops.block_buffers(x, mod, rope, work), run)
+    torch.cuda.synchronize()
+    for x in many:
+        assert torch.equal(x.view(torch.int16), one.view(torch.int16))
