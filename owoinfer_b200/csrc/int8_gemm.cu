@@ -947,8 +947,8 @@ int launch_kernel(const char* op, const b2_int8_operands* a, GemmParams p, cudaS
   return enqueue(op, kernel, grid, threads_of(kEpi, kBN, kW4), S::kSmemBytes, stream, kCtas, map_a, map_b, p);
 }
 
-// Tile choice: CTA pairs on 256 x 256 tiles when there are enough of them to fill the GPU; else one CTA per 128 x 256
-// tile, or 128 x 128 when even those leave SMs idle.
+// Tile choice of the W4A8 GEMM: CTA pairs on 256 x 256 tiles when there are enough of them to fill the GPU; else one CTA
+// per 128 x 256 tile, or 128 x 128 when even those leave SMs idle.
 int pick_tile(int tile, std::int64_t m, std::int64_t n_tiles_256) {
   if (tile != B2_TILE_AUTO) return tile;
   const std::int64_t pairs = ((m + 255) / 256) * n_tiles_256;
@@ -957,13 +957,41 @@ int pick_tile(int tile, std::int64_t m, std::int64_t n_tiles_256) {
   return big >= sm_count() ? B2_TILE_128x256 : B2_TILE_128x128;
 }
 
+// The same choice for an INT8 GEMM by what each shape takes, in units of 0.28 us (a CTA pair's time per K block): a launch
+// costs a fixed part (set-up, first loads, last epilogue) and one part per round of tiles over the SMs. Counting tiles alone
+// sent 800 rows x 3072 columns to two rounds of 128 x 128 tiles. Measured (N = 3072, weights from HBM, us):
+//   rows x K          128 x 128   128 x 256   pairs
+//   297 x 3072          12.1        17.8      16.0
+//   800 x 3072          18.5        17.7      16.2
+//   297 x 12288         30.5        49.0      36.6
+//   800 x 12288         54.8        47.8      36.8
+// QKV (9216 x 3072) on 297 rows: 19.0, 17.0, 15.6; SiTU-GLU (K = 3072) on 297 rows: F = 8192 31.0 (128 x 256), 27.3 (pairs);
+// F = 12288 34.1, 36.2.
+struct TileCost {
+  double fixed, per_block;
+};
+template <Epi kEpi>
+int pick_tile_int8(const GemmParams& p) {
+  constexpr bool kSitu = kEpi == Epi::kSituGlu;
+  constexpr TileCost kPair = kSitu ? TileCost{50, 1.1} : TileCost{33, 1.0}, kBig = kSitu ? TileCost{43, 1.64} : TileCost{27, 1.5}, kSmall{21, 0.95};
+  const int k_blocks = (p.k + kBK - 1) / kBK, sms = sm_count();
+  const std::int64_t m_tiles = (static_cast<std::int64_t>(p.m) + kBM - 1) / kBM, n128 = (static_cast<std::int64_t>(p.n) + 127) / 128;
+  const std::int64_t n256 = kSitu ? (p.half + 127) / 128 : (n128 + 1) / 2;
+  const auto cost = [&](const TileCost& c, std::int64_t tiles, int at_once) {
+    return c.fixed + c.per_block * static_cast<double>((tiles + at_once - 1) / at_once * k_blocks);
+  };
+  const double pair = cost(kPair, (m_tiles + 1) / 2 * n256, sms / 2), big = cost(kBig, m_tiles * n256, sms);
+  const double small = kSitu ? big : cost(kSmall, m_tiles * n128, sms);
+  return pair <= big && pair <= small ? B2_TILE_2CTA_256x256 : big <= small ? B2_TILE_128x256 : B2_TILE_128x128;
+}
+
 template <Epi kEpi>
 int dispatch(const char* op, const b2_int8_operands* a, const GemmParams& p, cudaStream_t stream, int tile) {
   if constexpr (kEpi == Epi::kSituGlu) {
-    const int t = pick_tile(tile, a->m, (p.half + 127) / 128);
+    const int t = tile != B2_TILE_AUTO ? tile : pick_tile_int8<kEpi>(p);
     return t == B2_TILE_2CTA_256x256 ? launch_kernel<256, kEpi, 2>(op, a, p, stream) : launch_kernel<256, kEpi, 1>(op, a, p, stream);
   } else {
-    const int t = pick_tile(tile, a->m, (a->n + 255) / 256);
+    const int t = tile != B2_TILE_AUTO ? tile : pick_tile_int8<kEpi>(p);
     if (t == B2_TILE_2CTA_256x256) return launch_kernel<256, kEpi, 2>(op, a, p, stream);
     return t == B2_TILE_128x256 ? launch_kernel<256, kEpi, 1>(op, a, p, stream) : launch_kernel<128, kEpi, 1>(op, a, p, stream);
   }

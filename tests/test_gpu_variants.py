@@ -107,3 +107,23 @@ def test_overlapping_launches_change_no_bit(ops, rows):
     torch.cuda.synchronize()
     for x in many:
         assert torch.equal(x.view(torch.int16), one.view(torch.int16))
+
+
+# Row counts on both sides of where the automatic choice changes: 128 x 128 tiles, 128 x 256 tiles, CTA pairs.
+@pytest.mark.parametrize("rows", [1, 128, 129, 256, 257, 385, 737, 769, 1281])
+def test_automatic_tile_gives_the_bits_of_every_tile(ops, rows):
+    g = torch.Generator("cuda").manual_seed(rows)
+    ints = lambda *s: torch.randint(-127, 128, s, dtype=torch.int8, device="cuda", generator=g)
+    for n, k in ((9216, 256), (1024, 3072)):
+        x, w = ints(rows, k), ints(n, k)
+        xs, ws = (torch.rand(s, device="cuda", generator=g) * 1e-3 for s in (rows, n))
+        gate, res = (torch.randn(s, device="cuda", generator=g).to(torch.bfloat16) for s in ((n,), (rows, n)))
+        forms = (lambda t: ops.int8_gemm(x, xs, w, ws, tile=t), lambda t: ops.int8_gemm_situ_glu(x, xs, w, ws, tile=t),
+                 lambda t: ops.int8_gemm_gated_residual(x, xs, w, ws, gate, res.clone(), tile=t))
+        for form in forms:
+            want = form(ops.TILE_AUTO).view(torch.int16)
+            for tile in (ops.TILE_128x128, ops.TILE_128x256, ops.TILE_2CTA_256x256):
+                assert torch.equal(form(tile).view(torch.int16), want)
+        acc = ops.int8_gemm_acc(x, w)
+        rows_ref = slice(0, min(rows, 8))
+        assert torch.equal(acc[rows_ref].double(), x[rows_ref].double() @ w.double().T)
