@@ -272,7 +272,10 @@ struct PrepArgs {
   // own0 = 0 and own1 is past every row.
   const __nv_bfloat16* slot[2];
   std::int64_t slot_ld, own0, own1;
-  __nv_bfloat16* tap;  // when set: a copy of the own rows' k | v, [own1 - own0, 2 heads 128]
+  __nv_bfloat16* tap;  // when set: a copy of the own rows' k | v, [own rows, 2 heads 128]
+  // When set: how many own rows there are, of which those that no query sequence covers ([cu[0], cu[batch]) are covered)
+  // get their QK-norm + RoPE and their place in the tap all the same. 0 = nobody reads them.
+  std::int64_t all_rows;
   // outputs
   std::int8_t* q_i8;
   std::int8_t* k_i8;
@@ -345,15 +348,48 @@ __device__ __forceinline__ void norm_rope_row(const std::uint32_t (&x)[4], const
   }
 }
 
+// The own rows ahead of the first and behind the last query sequence, numbered 0 .. `count` - 1.
+struct RowsOutside {
+  std::int64_t first, last, count;
+  __device__ __forceinline__ explicit RowsOutside(const PrepArgs& p)
+      : first(p.cu[0]), last(p.cu[p.batch]), count(p.all_rows - (last - first)) {}
+  __device__ __forceinline__ std::int64_t row(std::int64_t i) const { return i < first ? i : last + (i - first); }
+};
+
+// QK-norm + RoPE of the k rows outside the query sequences, by the CTAs of the first sequence (head h, 32 rows at a time).
+// Out of line: hardly a run has such rows, and the kernel's own registers stay what they were.
+__device__ __noinline__ void norm_rope_keys_outside(const PrepArgs& p, int bx, int h, int row, int lane) {
+  const RowsOutside outside(p);
+  const int pair = (lane & 7) * 8;
+  const std::uint32_t flip = lane < 8 ? 0x80008000u : 0u;
+  for (std::int64_t at = 32LL * bx; at < outside.count; at += 32LL * gridDim.x) {
+    const bool valid = at + row < outside.count;
+    const std::int64_t tok = outside.row(at + row);
+    __nv_bfloat16* k_at = p.k + tok * p.k_row + h * p.k_head + lane * 8;
+    const uint4 w = *reinterpret_cast<const uint4*>(p.k_norm + lane * 8);
+    uint4 k = make_uint4(0, 0, 0, 0), s = k, c = k;
+    if (valid) {
+      k = *reinterpret_cast<const uint4*>(k_at);
+      s = *reinterpret_cast<const uint4*>(p.table + tok * p.table_row + pair);
+      c = *reinterpret_cast<const uint4*>(p.table + tok * p.table_row + 64 + pair);
+    }
+    std::uint32_t y[4];
+    norm_rope_row({k.x, k.y, k.z, k.w}, {w.x, w.y, w.z, w.w}, {s.x ^ flip, s.y ^ flip, s.z ^ flip, s.w ^ flip},
+                  {c.x, c.y, c.z, c.w}, p.norm_factor, y);
+    if (valid) *reinterpret_cast<uint4*>(k_at) = make_uint4(y[0], y[1], y[2], y[3]);
+  }
+}
+
 // Fused prologue, one CTA per (32-token Q block, head, sequence): 32 token rows x 16 lanes x 8 channels. RMS-norm + RoPE
 // of q and k; Q quantised with the block's scale; k written back in place for the statistics and K/V quantisation
 // passes. Every load of a row is issued before the first use.
-__global__ void __launch_bounds__(512, 2) norm_rope_quant_q_kernel(const PrepArgs p) {
+__global__ void __launch_bounds__(512, 2) norm_rope_quant_q_kernel(const __grid_constant__ PrepArgs p) {
   dependents_may_start();
   wait_for_predecessors();
   const int bx = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int lane = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
   const int start = p.cu[b], len = p.cu[b + 1] - start;
+  if (b == 0 && p.all_rows > 0) norm_rope_keys_outside(p, bx, h, row, lane);
   const std::int64_t scale_at = (static_cast<std::int64_t>(b) * p.heads + h) * p.q_blocks + bx;
   if (bx * 32 >= len) {
     // A block at or past the sequence end holds no tokens: its scale is the empty block's.
@@ -552,6 +588,15 @@ __global__ void __launch_bounds__(256) quant_kv_kernel(const PrepArgs p) {
       __nv_bfloat16* at = p.tap + (tok[i] - p.own0) * 2 * width + h * kHeadDim + lane * 8;
       __stcs(reinterpret_cast<uint4*>(at), kr[i]);
       __stcs(reinterpret_cast<uint4*>(at + width), vr[i]);
+    }
+    if (b == 0 && p.all_rows > 0) {
+      const RowsOutside outside(p);  // (a tapped run reads no slots: its key rows are its own rows)
+      for (std::int64_t i = 16LL * bx + row; i < outside.count; i += 16LL * gridDim.x) {
+        const std::int64_t r = outside.row(i);
+        __nv_bfloat16* at = p.tap + r * 2 * width + h * kHeadDim + lane * 8;
+        *reinterpret_cast<uint4*>(at) = *reinterpret_cast<const uint4*>(p.k + r * p.k_row + h * p.k_head + lane * 8);
+        *reinterpret_cast<uint4*>(at + width) = *reinterpret_cast<const uint4*>(p.v + r * p.v_row + h * p.v_head + lane * 8);
+      }
     }
   }
   float mean[8], recp[8];
@@ -1382,6 +1427,7 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     p.slot[0] = static_cast<const __nv_bfloat16*>(rows->slot[0]), p.slot[1] = static_cast<const __nv_bfloat16*>(rows->slot[1]);
     p.slot_ld = rows->slot_ld, p.own0 = rows->own0, p.own1 = rows->own0 + total_q;
     p.tap = static_cast<__nv_bfloat16*>(rows->tap);
+    if (rows->slot_run || p.tap != nullptr) p.all_rows = total_q;
   }
   const dim3 stats_grid(l.chunks, static_cast<unsigned>(heads), batch);
   if (norm_rope != nullptr) {

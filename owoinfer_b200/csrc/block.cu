@@ -218,7 +218,7 @@ int b2_run_block_quant(const b2_block_weights* w, const b2_block_buffers* a, con
     }
     k0 = run->k0, k_rows = run->k1 - run->k0, cu_k = run->cu_seqlens_k;
     if (direct) {
-      rows.own0 = slot - k0, rows.slot_ld = slot_ld;
+      rows.own0 = slot - k0, rows.slot_ld = slot_ld, rows.slot_run = true;
       if (reads[0]) rows.slot[0] = static_cast<const __nv_bfloat16*>(run->slot_kv[0]) + k0 * slot_ld;
       if (reads[1]) rows.slot[1] = run->slot_kv[1];
     }

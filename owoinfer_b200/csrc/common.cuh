@@ -101,11 +101,13 @@ int prepare_situ_tables(cudaStream_t stream);
 
 // Key and value rows of an attention call beyond its k and v views. Rows [own0, own0 + q rows) of the views are the run's
 // own; the rows before and after them are read from slot[0] and slot[1] (bf16 rows k | v, 16-byte aligned, slot_ld
-// elements apart). tap, when set, receives a copy of the own k | v rows [q rows, 2 heads 128].
+// elements apart). tap, when set, receives a copy of the own k | v rows [q rows, 2 heads 128]. slot_run: the key sequences
+// have offsets of their own, so they may hold own rows that no query sequence does.
 struct AttentionRows {
   const void* slot[2];
   std::int64_t slot_ld, own0;
   void* tap;
+  bool slot_run;
 };
 int attention_rows(const b2_attention_options* o, const b2_view3* q, const b2_view3* k, const b2_view3* v, const b2_view3* out,
                    const std::int32_t* cu_q, const std::int32_t* cu_k, int batch, int max_seqlen, float scale, void* workspace,

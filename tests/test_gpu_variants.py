@@ -127,3 +127,43 @@ def test_automatic_tile_gives_the_bits_of_every_tile(ops, rows):
         acc = ops.int8_gemm_acc(x, w)
         rows_ref = slice(0, min(rows, 8))
         assert torch.equal(acc[rows_ref].double(), x[rows_ref].double() @ w.double().T)
+
+
+def test_rows_outside_the_sequences_are_tapped_and_read_as_keys(ops):
+    """cu_seqlens need not cover every row of a run. The tap still holds all rows, and key sequences of a run with slots may
+    reach rows that no query sequence covers: the same bits as with the separate QK-norm + RoPE and the copies."""
+    F, L, slot, lens = 512, 300, 70, [150, 87]
+    w = synth.block_weights(D, F, 31)
+    bw = ops.BlockWeights(w["norm1"], w["norm2"], w["q_norm"], w["k_norm"], w["qkv"], w["o"], w["up_gate"], w["down"])
+    mod, x0, rope = synth.modulation(D, 4), synth.activations(L, D, 9), ops.moss_rope_table(1, 1, L - 1)
+    cu = (synth.cu_seqlens(lens) + 13).contiguous()                      # rows 0..12 and 250..299 lie outside
+    inside = slice(13, 13 + sum(lens))
+
+    def run(max_len, **kw):
+        r = ops.block_run(L, cu, max_len, D=D, F=F, **kw)
+        ws = torch.zeros(ops.block_quant_workspace_bytes(r), dtype=torch.uint8, device="cuda")
+        x = x0.clone()
+        ops.run_block_quant(bw, ops.block_buffers(x, mod, rope, ws), r)
+        torch.cuda.synchronize()
+        return bits(x[inside])
+
+    xq, xs = ops.rotate_quantize(ops.rms_norm_modulate(x0, w["norm1"], mod[D:2 * D], mod[:D]))
+    qkv = ops.int8_gemm(xq, xs, w["qkv"][0], w["qkv"][1])
+    ops.qk_norm_rope_moss(qkv, H, w["q_norm"], w["k_norm"], rope)
+    plain = run(150)
+    for fused in (-1, 0):
+        tap = torch.zeros((L, 2 * D), dtype=torch.bfloat16, device="cuda")
+        assert np.array_equal(run(150, kv_tap=tap, fused_norm_rope=fused), plain)
+        assert np.array_equal(bits(tap), bits(qkv[:, D:]))
+
+    kv = torch.randn(slot * 2 * D + 8, device="cuda", generator=torch.Generator("cuda").manual_seed(7)).to(torch.bfloat16)
+    odd = torch.empty_like(kv)
+    odd[4:4 + slot * 2 * D] = kv[:slot * 2 * D]                          # only 8-byte aligned: the copies
+    aligned, shifted = kv[:slot * 2 * D].view(slot, 2 * D), odd[4:4 + slot * 2 * D].view(slot, 2 * D)
+    # Keys of the first sequence: slot A and own rows 0..162; of the second: own rows 163..299 and slot B.
+    both = dict(slot_rows=slot, cu_seqlens_k=synth.cu_seqlens([slot + 163, L - 163 + slot]), k0=0, k1=L + 2 * slot)
+    want = run(slot + 163, slot_kv=(shifted, shifted), **both)
+    assert np.array_equal(run(slot + 163, slot_kv=(aligned, aligned), **both), want)
+    assert np.array_equal(run(slot + 163, slot_kv=(aligned, aligned), fused_norm_rope=0, **both), want)
+    own = dict(slot_rows=slot, cu_seqlens_k=synth.cu_seqlens([163, L - 163]), k0=slot, k1=slot + L)   # neither slot read
+    assert np.array_equal(run(163, slot_kv=(None, None), **own), run(163, slot_kv=(None, None), fused_norm_rope=0, **own))
