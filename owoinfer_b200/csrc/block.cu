@@ -101,6 +101,37 @@ int site_operands(const char* op, const b2_linear& lin, int tier, std::int8_t* w
 }
 
 }  // namespace
+
+int check_block_after_tap(const b2_block_weights* w, const b2_block_run* run_in) {
+  constexpr const char* op = "run_block_quant";
+  if (const int rc = check_run(op, run_in)) return rc;
+  const b2_block_run run = whole_run(run_in);
+  b2_attention_options ao = run.attention;
+  if (ao.variant == 0) ao.variant = B2_ATTENTION_Q8_FP8_F32ACC;
+  // No row: the checks run, nothing is launched. `any` stands for the activations, which the block places itself.
+  alignas(16) static const unsigned char any[16] = {};
+  auto* at = const_cast<unsigned char*>(any);
+  const b2_view3 none{at, 0, run.heads, 3 * run.D, 128};
+  if (const int rc = b2_attention_q8(&ao, &none, &none, &none, &none, run.cu_seqlens, run.cu_seqlens, run.batch, run.max_seqlen, 1.f,
+                                     nullptr, 0, nullptr, nullptr)) {
+    return rc;
+  }
+  if (!aligned_to(w->norm2, 16)) return fail_invalid(op, "norm weights must be 16-byte aligned");
+  const auto site = [&](const b2_linear& lin, std::int64_t n, std::int64_t k, int epilogue) -> int {
+    if (run.tier == B2_TIER_W4A8) {
+      if (lin.w4 == nullptr) return fail_invalid(op, "missing grouped 4-bit weight");
+      return b2_w4a8_gemm(nullptr, k, nullptr, lin.w4, 0, n, k, epilogue, at, at, epilogue == 2 ? n / 2 : n, reinterpret_cast<std::int8_t*>(at), nullptr);
+    }
+    if (lin.w == nullptr || lin.scale == nullptr) return fail_invalid(op, "missing INT8 or INT4 weight");
+    const b2_int8_operands o{nullptr, k, nullptr, lin.w, lin.scale, 0, n, k};
+    if (epilogue == 1) return b2_int8_gemm_gated_residual(&o, nullptr, at, at, n, nullptr, B2_TILE_AUTO);
+    return b2_int8_gemm_situ_glu(&o, at, n / 2, nullptr, B2_TILE_AUTO);
+  };
+  if (const int rc = site(w->o, run.D, run.D, 1)) return rc;
+  if (const int rc = site(w->up_gate, 2 * run.F, run.D, 2)) return rc;
+  return site(w->down, run.D, run.F, 1);
+}
+
 }  // namespace b2
 
 using namespace b2;

@@ -99,6 +99,10 @@ int gemm_site(const b2_int8_operands* o, int epilogue, const void* aux, void* ou
 // afterwards. For callers that are about to capture: inside a capture every SiTU-GLU launch would bring a fill along.
 int prepare_situ_tables(cudaStream_t stream);
 
+// What a block run refuses after its tap (attention options, the weights of o, up_gate and down), for a caller that ends a
+// block at the tap but refuses what a whole block would. Launches nothing.
+int check_block_after_tap(const b2_block_weights* w, const b2_block_run* run);
+
 // Key and value rows of an attention call beyond its k and v views. Rows [own0, own0 + q rows) of the views are the run's
 // own; the rows before and after them are read from slot[0] and slot[1] (bf16 rows k | v, 16-byte aligned, slot_ld
 // elements apart). tap, when set, receives a copy of the own k | v rows [q rows, 2 heads 128]. slot_run: the key sequences

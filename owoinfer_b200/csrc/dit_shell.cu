@@ -953,6 +953,8 @@ int prefill_impl(const b2_dit_model* model, const b2_prefill* prefill, void* str
   if (f.workspace == nullptr || !aligned_to(f.workspace, 256) || f.workspace_bytes < c.total) {
     return fail_invalid(op, "workspace must be 256-byte aligned and hold b2_dit_prefill_workspace_bytes() = " + std::to_string(c.total));
   }
+  // The last block ends at its tap below; a model that lacks what follows is refused all the same.
+  if (const int rc = check_block_after_tap(&m.blocks[m.num_blocks - 1], &run)) return rc;
   cudaStream_t stream = as_stream(stream_);
   const LaunchChain chain(stream);
   const std::int64_t D = m.D;

@@ -238,6 +238,33 @@ def test_block_rejects_mismatched_buffers():
     assert _status(lib.b2_run_block_quant(C.byref(w), C.byref(b), C.byref(run), None))[0] == -1
 
 
+@pytest.mark.parametrize("tier", [0, 1, 2])
+@pytest.mark.parametrize("lack", ["o", "up_gate", "down", "variant"])
+def test_prefill_refuses_a_last_block_that_could_not_run(tier, lack):
+    """The prefill ends its last block at the tap. What the rest of that block refuses stays refused, before any launch."""
+    lib = _lib.lib()
+    at = 0x10000
+    w4 = _lib.W4Weight(packed=at, s_rel=at, scale_kind=0, group=64, codebook=None, s_channel=at)
+    lin = lambda: _lib.Linear(w=at, scale=at, w4=C.pointer(w4))
+    blocks = (_lib.BlockWeights * 1)()
+    b = blocks[0]
+    b.struct_size, b.norm1, b.norm2, b.q_norm, b.k_norm = C.sizeof(_lib.BlockWeights), at, at, at, at
+    for name in ("qkv", "o", "up_gate", "down"):
+        setattr(b, name, _lib.Linear() if name == lack else lin())
+    m = _lib.DitModel()
+    m.struct_size, m.blocks, m.num_blocks, m.D, m.F, m.heads, m.latent_channels = C.sizeof(_lib.DitModel), blocks, 1, 3072, 512, 24, 128
+    m.block_mod_w = m.block_mod_bias = m.video_w = m.video_bias = at
+    ptrs, side = (C.c_void_p * 1)(at), (C.c_int * 1)(4)
+    f = _lib.Prefill()
+    f.struct_size, f.latents, f.heights, f.widths, f.num_refs = C.sizeof(_lib.Prefill), ptrs, side, side, 1
+    f.time_vector, f.kv_out, f.tier, f.workspace = at, at, tier, at
+    f.attention = _lib.AttentionOptions(1 if lack == "variant" else 3, 0.0, 0.0)
+    f.workspace_bytes = lib.b2_dit_prefill_workspace_bytes(C.byref(m), C.byref(f))
+    assert f.workspace_bytes > 0
+    rc, msg = _status(lib.b2_dit_prefill_references(C.byref(m), C.byref(f), None))
+    assert (rc, "only the e4m3" in msg) == (-3, True) if lack == "variant" else (rc, "missing" in msg) == (-1, True)
+
+
 def test_step_graph_cache_handle_and_checks():
     """A cache is host state until its first forward; a graphed forward is refused on the default stream and on a bad
     forward before anything is enqueued (dit_graph.h:49-52: the stream of a capture is not the default stream)."""
