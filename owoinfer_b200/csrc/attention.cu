@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <limits>
 #include <string>
 
 #include "common.cuh"
@@ -268,8 +269,8 @@ struct PrepArgs {
   std::int64_t table_row;
   float norm_factor;
   // Keys and values that live elsewhere (a block run over cached reference rows): key rows [own0, own1) are rows of k / v,
-  // the rows before and after them rows of slot[0] and slot[1] (k | v side by side, slot_ld elements apart). Without slots
-  // own0 = 0 and own1 is past every row.
+  // the rows before and after them rows of slot[0] and slot[1] (k | v side by side, slot_ld elements apart). Without a slot
+  // behind them own1 is past every row, without one ahead of them own0 = 0.
   const __nv_bfloat16* slot[2];
   std::int64_t slot_ld, own0, own1;
   __nv_bfloat16* tap;  // when set: a copy of the own rows' k | v, [own rows, 2 heads 128]
@@ -581,16 +582,17 @@ __global__ void __launch_bounds__(256) quant_kv_kernel(const PrepArgs p) {
   }
   if (p.tap != nullptr) {
     // The rows pass through these registers anyway: a copy of the whole k | v matrix of its own would read them once more.
+    // (A tapped run reads no slots: its key rows are its own rows.)
     const std::int64_t width = static_cast<std::int64_t>(p.heads) * kHeadDim;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      if (!valid[i] || tok[i] < p.own0 || tok[i] >= p.own1) continue;
-      __nv_bfloat16* at = p.tap + (tok[i] - p.own0) * 2 * width + h * kHeadDim + lane * 8;
+      if (!valid[i] || tok[i] >= p.all_rows) continue;
+      __nv_bfloat16* at = p.tap + tok[i] * 2 * width + h * kHeadDim + lane * 8;
       __stcs(reinterpret_cast<uint4*>(at), kr[i]);
       __stcs(reinterpret_cast<uint4*>(at + width), vr[i]);
     }
-    if (b == 0 && p.all_rows > 0) {
-      const RowsOutside outside(p);  // (a tapped run reads no slots: its key rows are its own rows)
+    if (b == 0) {
+      const RowsOutside outside(p);
       for (std::int64_t i = 16LL * bx + row; i < outside.count; i += 16LL * gridDim.x) {
         const std::int64_t r = outside.row(i);
         __nv_bfloat16* at = p.tap + r * 2 * width + h * kHeadDim + lane * 8;
@@ -1422,10 +1424,11 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   p.v_recp = reinterpret_cast<float*>(base + l.v_recp);
   p.part_sum = reinterpret_cast<float*>(base + l.part_sum);
   p.part_amax = reinterpret_cast<float*>(base + l.part_amax);
-  p.own1 = total_k;
+  p.own1 = std::numeric_limits<std::int64_t>::max();
   if (rows != nullptr) {
     p.slot[0] = static_cast<const __nv_bfloat16*>(rows->slot[0]), p.slot[1] = static_cast<const __nv_bfloat16*>(rows->slot[1]);
-    p.slot_ld = rows->slot_ld, p.own0 = rows->own0, p.own1 = rows->own0 + total_q;
+    p.slot_ld = rows->slot_ld, p.own0 = rows->own0;
+    if (p.slot[1] != nullptr) p.own1 = rows->own0 + total_q;
     p.tap = static_cast<__nv_bfloat16*>(rows->tap);
     if (rows->slot_run || p.tap != nullptr) p.all_rows = total_q;
   }
