@@ -277,6 +277,7 @@ struct PrepArgs {
   // When set: how many own rows there are, of which those that no query sequence covers ([cu[0], cu[batch]) are covered)
   // get their QK-norm + RoPE and their place in the tap all the same. 0 = nobody reads them.
   std::int64_t all_rows;
+  std::int64_t key_rows;  // rows of the K and V views (the quantised copies have as many)
   // outputs
   std::int8_t* q_i8;
   std::int8_t* k_i8;
@@ -564,6 +565,12 @@ __global__ void __launch_bounds__(256) quant_kv_kernel(const PrepArgs p) {
   const int lane = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
   const int start = p.cu[b], len = p.cu[b + 1] - start;
   const std::int64_t stat = (static_cast<std::int64_t>(b) * p.heads + h) * kHeadDim + lane * 8;
+  if (bx == 0 && b == p.batch - 1) {
+    // Rows behind the last sequence that its last 128-key tile brings along: their P is zero, but a NaN that the workspace
+    // held there would make it through the product.
+    const std::int64_t end = static_cast<std::int64_t>(start) + len, stop = min(end + 127, p.key_rows);
+    for (std::int64_t r = end + row; r < stop; r += 16) *reinterpret_cast<uint2*>(p.v8 + (r * p.heads + h) * kHeadDim + lane * 8) = make_uint2(0u, 0u);
+  }
   uint4 kr[4], vr[4];
   bool valid[4];
   std::int64_t tok[4];
@@ -1424,6 +1431,7 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   p.v_recp = reinterpret_cast<float*>(base + l.v_recp);
   p.part_sum = reinterpret_cast<float*>(base + l.part_sum);
   p.part_amax = reinterpret_cast<float*>(base + l.part_amax);
+  p.key_rows = total_k;
   p.own1 = std::numeric_limits<std::int64_t>::max();
   if (rows != nullptr) {
     p.slot[0] = static_cast<const __nv_bfloat16*>(rows->slot[0]), p.slot[1] = static_cast<const __nv_bfloat16*>(rows->slot[1]);

@@ -167,3 +167,21 @@ def test_rows_outside_the_sequences_are_tapped_and_read_as_keys(ops):
     assert np.array_equal(run(slot + 163, slot_kv=(aligned, aligned), fused_norm_rope=0, **both), want)
     own = dict(slot_rows=slot, cu_seqlens_k=synth.cu_seqlens([163, L - 163]), k0=slot, k1=slot + L)   # neither slot read
     assert np.array_equal(run(163, slot_kv=(None, None), **own), run(163, slot_kv=(None, None), fused_norm_rope=0, **own))
+
+
+def test_key_rows_past_the_last_sequence_do_not_reach_the_output(ops):
+    """The last key tile of the last sequence may hold rows that no sequence covers; whatever the workspace holds there
+    (here NaN bytes) has no part in the output."""
+    lens, extra = [70, 200], 61
+    total = sum(lens)
+    g = torch.Generator("cuda").manual_seed(3)
+    q = torch.randn((total, 2, 128), device="cuda", generator=g).to(torch.bfloat16)
+    k, v = (torch.randn((total + extra, 2, 128), device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    cu, outs = synth.cu_seqlens(lens), []
+    for rows in (total, total + 1, total + extra):
+        ws = torch.full((ops.attention_q8_workspace_bytes(total, rows, 2, 200, 2),), 0x7f, dtype=torch.uint8, device="cuda")
+        out = torch.zeros_like(q)
+        ops.attention_q8(q, k[:rows], v[:rows], out, cu, cu, 200, ops.SM_SCALE, workspace=ws)
+        torch.cuda.synchronize()
+        outs.append(bits(out))
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
