@@ -1187,7 +1187,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       const float inv_d = rcp_approx(d_run);
       const int row = q0 + r_local;
       __nv_bfloat16* orow = a.out + static_cast<std::int64_t>(q_start + row) * a.out_row + h * a.out_head;
-      const float* vs = a.v_scale + sc_base * kHeadDim;
+      const float* vs = a.v_scale + sc_base * kHeadDim;  // written by this call: ordinary loads (see wait_for_predecessors)
 #pragma unroll 1
       for (int cc = 0; cc < 4; ++cc) {
         std::uint32_t r[32];
@@ -1196,9 +1196,12 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         if (row < qo_len) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
+            const float4 s0 = *reinterpret_cast<const float4*>(vs + cc * 32 + 8 * v);
+            const float4 s1 = *reinterpret_cast<const float4*>(vs + cc * 32 + 8 * v + 4);
+            const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
             float o[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[8 * v + i]) * inv_d * __ldg(vs + cc * 32 + 8 * v + i);
+            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[8 * v + i]) * inv_d * s[i];
             *reinterpret_cast<uint4*>(orow + cc * 32 + 8 * v) =
                 make_uint4(pack_bf2(o[0], o[1]), pack_bf2(o[2], o[3]), pack_bf2(o[4], o[5]), pack_bf2(o[6], o[7]));
           }

@@ -160,7 +160,10 @@ __device__ __forceinline__ std::uint32_t smem_u32(const void* p) {
   return static_cast<std::uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Programmatic dependent launch (see LaunchChain): both are no-ops in a kernel launched the ordinary way.
+// Programmatic dependent launch (see LaunchChain): both are no-ops in a kernel launched the ordinary way. A kernel may be
+// resident while kernels before it in its chain still write, and the wait orders ordinary loads only: what a kernel of the
+// same chain may write is never read with __ldg or any other read-only-cache load, which is for data that is constant
+// for the whole call (weights and their scales, norm weights, tables filled by an earlier call).
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -159,7 +159,7 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int* 
 // One SiTU factor of the bf16 value with these bits from the full table in global memory (the slow path for a value
 // outside the shared-memory slice; same entries, so the same bits either way).
 __device__ __forceinline__ float situ_factor_full(const std::uint16_t* full, std::uint32_t bits) {
-  return __uint_as_float(static_cast<std::uint32_t>(__ldg(full + bits)) << 16);
+  return __uint_as_float(static_cast<std::uint32_t>(full[bits]) << 16);
 }
 
 // kCtas == 2: a CTA pair shares one 256 x 256 tile; each CTA stages its 128 rows of A and 128 of the 256 rows of B.
@@ -278,7 +278,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const bool gate = i < kMiniGate;
       const std::uint32_t j = gate ? i : i - kMiniGate;  // [sign (gate only)][exponent][mantissa]
       const std::uint32_t bits = ((j >> 12) << 15) | ((((j >> 7) & 31u) + kMiniExpLo) << 7) | (j & 127u);
-      s_tab[i] = __ldg((gate ? p.t_gate : p.t_hidden) + bits);
+      s_tab[i] = (gate ? p.t_gate : p.t_hidden)[bits];  // (ordinary loads: the chain itself may have filled the tables)
     }
   }
   tc_fence_before();
@@ -554,8 +554,9 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               }
             }
             if constexpr (kEpi == Epi::kGatedResidual) {
-              // The gate stays packed bf16 (two words for these four columns): the epilogue multiplies packed pairs.
-              const uint2 raw = __ldg(reinterpret_cast<const uint2*>(p.gate + col));
+              // The gate stays packed bf16 (two words for these four columns): the epilogue multiplies packed pairs. An
+              // ordinary load: a forward computes its gates in the same chain of launches.
+              const uint2 raw = *reinterpret_cast<const uint2*>(p.gate + col);
               g = make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y), 0.f, 0.f);
             }
           }

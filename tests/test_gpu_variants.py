@@ -185,3 +185,114 @@ def test_key_rows_past_the_last_sequence_do_not_reach_the_output(ops):
         torch.cuda.synchronize()
         outs.append(bits(out))
     assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+
+
+class Serial:
+    """A block call by call through the separate public ops, synchronised after each: no launch overlaps another one's
+    call. (The launches inside one attention call still overlap; those are held to the oracle elsewhere.)"""
+
+    def __init__(self, ops, tier, w, F):
+        self.o, self.tier, self.w, self.F = ops, tier, w, F
+        self.packed = {n: ops.make_w4(w[n][0], w[n][1], 64, w[n][2]) if tier == ops.TIER_W4A8 else w[n] for n in ("qkv", "o", "up_gate", "down")}
+        self.block = ops.BlockWeights(w["norm1"], w["norm2"], w["q_norm"], w["k_norm"], *self.packed.values())
+
+    def do(self, f, *a, **kw):
+        out = f(*a, **kw)
+        torch.cuda.synchronize()
+        return out
+
+    def quant(self, x, *norm):
+        if self.tier != self.o.TIER_W4A4_VIA_INT8:
+            return self.do(self.o.rms_norm_modulate_rotate_quantize if norm else self.o.rotate_quantize, x, *norm)
+        q, s = self.do(self.o.rms_norm_modulate_convrot_quantize_int4 if norm else self.o.convrot_quantize_int4, x, *norm)
+        return self.do(self.o.unpack_int4, q), s
+
+    def site(self, name, xq, xs, epilogue, gate=None, res=None):
+        o, lin = self.o, self.packed[name]
+        if self.tier == o.TIER_W4A8:
+            return self.do(o.w4a8_gemm, xq, xs, lin, self.w[name][0].shape[0], epilogue, gate, res)
+        w, s = (lin[0] if self.tier == o.TIER_INT8 else self.do(o.unpack_int4, lin[0])), lin[1]
+        if epilogue == 1:
+            return self.do(o.int8_gemm_gated_residual, xq, xs, w, s, gate, res)
+        return self.do(o.int8_gemm if epilogue == 0 else o.int8_gemm_situ_glu, xq, xs, w, s)
+
+    def __call__(self, x, mod, rope, cu, max_len, slots=None, cu_k=None):
+        """x in place; slots: (slot A, slot B) rows k | v. Returns the k | v rows of the run (the tap)."""
+        o, w, m, L = self.o, self.w, [mod[i * D:(i + 1) * D] for i in range(6)], x.shape[0]
+        qkv = self.site("qkv", *self.quant(x, w["norm1"], m[1], m[0]), 0)
+        self.do(o.qk_norm_rope_moss, qkv, H, w["q_norm"], w["k_norm"], rope)
+        kv = qkv[:, D:]
+        if slots is not None:
+            kv = torch.cat([slots[0], kv, slots[1]])
+        heads = lambda t, at: t.as_strided((t.shape[0], H, 128), (t.stride(0), 128, 1), t.storage_offset() + at)
+        attn = torch.empty((L, D), dtype=torch.bfloat16, device="cuda")
+        self.do(o.attention_q8, heads(qkv, 0), heads(kv, 0), heads(kv, D), attn.view(L, H, 128), cu, cu if cu_k is None else cu_k, max_len, o.SM_SCALE)
+        self.site("o", *self.quant(attn), 1, m[2], x)
+        ffn = self.site("up_gate", *self.quant(x, w["norm2"], m[4], m[3]), 2)
+        self.site("down", *self.quant(ffn), 1, m[5], x)
+        return qkv[:, D:].contiguous()
+
+
+@pytest.fixture(scope="module")
+def serial_blocks(ops):
+    F = 1024
+    return {t: [Serial(ops, t, synth.block_weights(D, F, 70 + 10 * i, tier=t), F) for i in range(2)]
+            for t in (ops.TIER_INT8, ops.TIER_W4A4_VIA_INT8, ops.TIER_W4A8)}
+
+
+@pytest.mark.parametrize("tier", [0, 1, 2])
+@pytest.mark.parametrize("rows", [33, 512, 513])   # the tensor-core kernels let their successor start early up to 512 rows
+def test_a_step_of_overlapping_launches_equals_its_calls_one_by_one(ops, serial_blocks, tier, rows):
+    """Two blocks in one chain of launches, eagerly and replayed from a graph, against every call by itself."""
+    blocks = serial_blocks[tier]
+    lens = [rows - rows // 3, rows // 3]
+    mod, rope, x0 = synth.modulation(D, 4), ops.moss_rope_table(1, 1, rows - 1), synth.activations(rows, D, 9)
+    cu = synth.cu_seqlens(lens)
+    want = x0.clone()
+    for b in blocks:
+        b(want, mod, rope, cu, lens[0])
+    run = ops.block_run(rows, cu, lens[0], D=D, F=blocks[0].F, tier=tier)
+    work = torch.empty(ops.block_quant_workspace_bytes(run), dtype=torch.uint8, device="cuda")
+    x = x0.clone()
+    step = lambda: ops.dit_step([b.block for b in blocks], ops.block_buffers(x, mod, rope, work), run)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for go in (step, graph.replay):
+        for _ in range(4):
+            work.fill_(0x7f)                        # a value read before it is written shows
+            x.copy_(x0)
+            go()
+            torch.cuda.synchronize()
+            assert torch.equal(x.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("tier", [0, 1, 2])
+@pytest.mark.parametrize("n0,n1", [(20, 13), (300, 333)])
+def test_taps_and_slots_in_a_chain_equal_the_calls_one_by_one(ops, serial_blocks, tier, n0, n1):
+    b, slot, L = serial_blocks[tier][0], 65, n0 + n1
+    mod, rope, x0 = synth.modulation(D, 4), ops.moss_rope_table(1, 1, L - 1), synth.activations(L, D, 9)
+    cu, kv = synth.cu_seqlens([n0, n1]), torch.randn((2, slot, 2 * D), device="cuda", generator=torch.Generator("cuda").manual_seed(n0)).to(torch.bfloat16)
+
+    def chain(**kw):
+        r = ops.block_run(L, cu, max(n0, n1) + slot, D=D, F=b.F, tier=tier, **kw)
+        x, work = x0.clone(), torch.full((ops.block_quant_workspace_bytes(r),), 0x7f, dtype=torch.uint8, device="cuda")
+        ops.run_block_quant(b.block, ops.block_buffers(x, mod, rope, work), r)
+        torch.cuda.synchronize()
+        return bits(x)
+
+    want, tap = x0.clone(), torch.zeros((L, 2 * D), dtype=torch.bfloat16, device="cuda")
+    rows = b(want, mod, rope, cu, max(n0, n1) + slot)
+    assert np.array_equal(chain(kv_tap=tap), bits(want)) and np.array_equal(bits(tap), bits(rows))
+    # Both slots; then key rows that begin (and end) inside the run's own rows, which keep the copies.
+    want, cu_k = x0.clone(), synth.cu_seqlens([slot + n0, n1 + slot])
+    b(want, mod, rope, cu, max(n0, n1) + slot, slots=kv, cu_k=cu_k)
+    assert np.array_equal(chain(slot_rows=slot, slot_kv=(kv[0], kv[1]), cu_seqlens_k=cu_k, k0=0, k1=L + 2 * slot), bits(want))
+    want, cut = x0.clone(), 5
+    b(want, mod, rope, cu, max(n0, n1) + slot, slots=(kv[0], kv[1]), cu_k=synth.cu_seqlens([n0 - cut, n1 + slot]) + slot + cut)
+    got = chain(slot_rows=slot, slot_kv=(None, kv[1]), cu_seqlens_k=synth.cu_seqlens([n0 - cut, n1 + slot]), k0=slot + cut, k1=L + 2 * slot)
+    assert np.array_equal(got, bits(want))
+    want = x0.clone()
+    b(want, mod, rope, cu, max(n0, n1) + slot, slots=(kv[0], kv[1]), cu_k=synth.cu_seqlens([slot + n0, n1 - cut]))
+    got = chain(slot_rows=slot, slot_kv=(kv[0], None), cu_seqlens_k=synth.cu_seqlens([slot + n0, n1 - cut]), k0=0, k1=slot + L - cut)
+    assert np.array_equal(got, bits(want))
