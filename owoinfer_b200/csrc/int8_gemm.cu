@@ -98,8 +98,9 @@ struct GemmParams {
 };
 
 __device__ int g_gemm_status = 0;  // set to 1 by a CTA whose bounded wait expired
-// How long a wait on an mbarrier may last. A step never comes near it (the longest wait of a healthy launch is one K
-// loop, tens of microseconds); an operator does not notice it.
+// How long a wait on an mbarrier may last. A step never comes near it (every role that waits has waited for the kernels
+// before this one first, so the longest wait of a healthy launch is one K loop, tens of microseconds); an operator does not
+// notice it.
 __device__ unsigned long long g_gemm_wait_limit_ns = 200000000ull;
 // Test hook: 1 = the TMA warp of every CTA leaves out the loads of the last K block of its first tile, so that the
 // stage's barrier never completes and the bounded waits run out.
@@ -379,6 +380,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // The whole warp of the issuing CTA walks the loop (uniform control flow, so descriptors and loop state stay in
     // uniform registers; every lane takes the waits); one elected lane issues the MMAs and commits.
     if (rank == 0) {
+      wait_for_predecessors();  // (so that the time limit of the waits below counts from here; the operands come later still)
       constexpr std::uint32_t idesc = umma_idesc(/*s32*/ 2, /*s8*/ 1, /*s8*/ 1, 0, 0, kBM * kCtas, kBN);
       constexpr std::uint32_t kStageUnits = S::kStageBytes >> 4;  // descriptor address units are 16 bytes
       const std::uint64_t da0 = umma_desc_sw128(a_addr(0)), db0 = umma_desc_sw128(b_addr(0));
