@@ -1453,7 +1453,8 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     p.norm_factor = static_cast<float>(norm_rows) / static_cast<float>(norm_rows * kHeadDim);
     PrepArgs own = p;  // queries and the key rows of the same tokens
     own.cu = cu_seqlens_q, own.k = p.k + p.own0 * p.k_row;
-    if (const int rc = enqueue(op, norm_rope_quant_q_kernel, dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st, 1, own)) return rc;
+    const auto kernel = p.all_rows > 0 ? norm_rope_quant_q_kernel<true> : norm_rope_quant_q_kernel<false>;
+    if (const int rc = enqueue(op, kernel, dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st, 1, own)) return rc;
   }
   if (const int rc = enqueue(op, stats_kernel, stats_grid, 256, 0, st, 1, p)) return rc;
   if (const int rc = enqueue(op, finalize_kernel, dim3(static_cast<unsigned>(heads), batch), kHeadDim, 0, st, 1, p)) return rc;

@@ -274,12 +274,21 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   }
   if constexpr (kEpi == Epi::kSituGlu) {
-    if (p.early_tables == 0) wait_for_predecessors();
-    for (int i = threadIdx.x; i < kMiniGate + kMiniHidden; i += blockDim.x) {
-      const bool gate = i < kMiniGate;
-      const std::uint32_t j = gate ? i : i - kMiniGate;  // [sign (gate only)][exponent][mantissa]
-      const std::uint32_t bits = ((j >> 12) << 15) | ((((j >> 7) & 31u) + kMiniExpLo) << 7) | (j & 127u);
-      s_tab[i] = (gate ? p.t_gate : p.t_hidden)[bits];  // (ordinary loads: the chain itself may have filled the tables)
+    const auto fill = [&](auto load) {
+      for (int i = threadIdx.x; i < kMiniGate + kMiniHidden; i += blockDim.x) {
+        const bool gate = i < kMiniGate;
+        const std::uint32_t j = gate ? i : i - kMiniGate;  // [sign (gate only)][exponent][mantissa]
+        const std::uint32_t bits = ((j >> 12) << 15) | ((((j >> 7) & 31u) + kMiniExpLo) << 7) | (j & 127u);
+        s_tab[i] = load((gate ? p.t_gate : p.t_hidden) + bits);
+      }
+    };
+    // Tables of an earlier call are constant: the read-only cache's loads run ahead of the shared stores. Tables that this
+    // very chain of launches fills are not.
+    if (p.early_tables != 0) {
+      fill([](const std::uint16_t* at) { return __ldg(at); });
+    } else {
+      wait_for_predecessors();
+      fill([](const std::uint16_t* at) { return *at; });
     }
   }
   tc_fence_before();
