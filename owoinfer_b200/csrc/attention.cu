@@ -359,9 +359,7 @@ struct RowsOutside {
 };
 
 // QK-norm + RoPE of the k rows outside the query sequences, by the CTAs of the first sequence (head h, 32 rows at a time).
-// Out of line: hardly a run has such rows, and the kernel's own registers stay what they were.
-__device__ __noinline__ void norm_rope_keys_outside(const PrepArgs& p, int bx, int h, int row, int lane) {
-  const RowsOutside outside(p);
+__device__ __forceinline__ void norm_rope_keys_outside(const PrepArgs& p, const RowsOutside& outside, int bx, int h, int row, int lane) {
   const int pair = (lane & 7) * 8;
   const std::uint32_t flip = lane < 8 ? 0x80008000u : 0u;
   for (std::int64_t at = 32LL * bx; at < outside.count; at += 32LL * gridDim.x) {
@@ -384,14 +382,18 @@ __device__ __noinline__ void norm_rope_keys_outside(const PrepArgs& p, int bx, i
 
 // Fused prologue, one CTA per (32-token Q block, head, sequence): 32 token rows x 16 lanes x 8 channels. RMS-norm + RoPE
 // of q and k; Q quantised with the block's scale; k written back in place for the statistics and K/V quantisation
-// passes. Every load of a row is issued before the first use.
-__global__ void __launch_bounds__(512, 2) norm_rope_quant_q_kernel(const __grid_constant__ PrepArgs p) {
+// passes. Every load of a row is issued before the first use. kAllRows: the rows outside the sequences too (p.all_rows).
+template <bool kAllRows>
+__global__ void __launch_bounds__(512, 2) norm_rope_quant_q_kernel(const PrepArgs p) {
   dependents_may_start();
   wait_for_predecessors();
   const int bx = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int lane = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
   const int start = p.cu[b], len = p.cu[b + 1] - start;
-  if (b == 0 && p.all_rows > 0) norm_rope_keys_outside(p, bx, h, row, lane);
+  if constexpr (kAllRows) {
+    const RowsOutside outside(p);
+    if (b == 0) norm_rope_keys_outside(p, outside, bx, h, row, lane);
+  }
   const std::int64_t scale_at = (static_cast<std::int64_t>(b) * p.heads + h) * p.q_blocks + bx;
   if (bx * 32 >= len) {
     // A block at or past the sequence end holds no tokens: its scale is the empty block's.
@@ -1192,16 +1194,17 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       for (int cc = 0; cc < 4; ++cc) {
         std::uint32_t r[32];
         tmem_ld_32x32(tmem_o + lane_off + cc * 32, r);
+        float4 s[8];  // all of the part's scales ahead of its stores, which ordinary loads cannot pass
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i] = *reinterpret_cast<const float4*>(vs + cc * 32 + 4 * i);
         tmem_ld_wait();
         if (row < qo_len) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            const float4 s0 = *reinterpret_cast<const float4*>(vs + cc * 32 + 8 * v);
-            const float4 s1 = *reinterpret_cast<const float4*>(vs + cc * 32 + 8 * v + 4);
-            const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+            const float sv[8] = {s[2 * v].x, s[2 * v].y, s[2 * v].z, s[2 * v].w, s[2 * v + 1].x, s[2 * v + 1].y, s[2 * v + 1].z, s[2 * v + 1].w};
             float o[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[8 * v + i]) * inv_d * s[i];
+            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[8 * v + i]) * inv_d * sv[i];
             *reinterpret_cast<uint4*>(orow + cc * 32 + 8 * v) =
                 make_uint4(pack_bf2(o[0], o[1]), pack_bf2(o[2], o[3]), pack_bf2(o[4], o[5]), pack_bf2(o[6], o[7]));
           }
