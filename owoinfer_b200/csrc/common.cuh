@@ -160,6 +160,38 @@ __device__ __forceinline__ std::uint32_t smem_u32(const void* p) {
   return static_cast<std::uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Grouped 4-bit weights: value = clamp(rint(level[code] * group scale), +-127); zero where the scale is NaN or negative.
+// ---------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ float e4m3_value(std::uint32_t b) {
+  const std::uint32_t e = (b >> 3) & 0xF, mant = b & 7;
+  float mag;
+  if (e == 0xF && mant == 7) mag = __int_as_float(0x7FC00000);
+  else if (e == 0) mag = static_cast<float>(mant) * 0.001953125f;  // 2^-9
+  else mag = __uint_as_float(((e + 120u) << 23) | (mant << 20));
+  return (b & 0x80) ? -mag : mag;
+}
+__device__ __forceinline__ std::uint32_t w4_byte(float level, float scale) {
+  return static_cast<std::uint32_t>(static_cast<int>(fminf(127.f, fmaxf(-127.f, rintf(fmul(level, scale)))))) & 0xFFu;
+}
+// The values of all 16 codes under one scale: code c in byte c % 4 of word c / 4.
+template <typename Level>
+__device__ __forceinline__ uint4 w4_table(float scale, const Level& level) {
+  std::uint32_t t[4] = {0u, 0u, 0u, 0u};
+  if (!(isnan(scale) || scale < 0.0f)) {
+#pragma unroll
+    for (int c = 0; c < 16; ++c) t[c >> 2] |= w4_byte(level(c), scale) << (8 * (c & 3));
+  }
+  return make_uint4(t[0], t[1], t[2], t[3]);
+}
+// Eight 4-bit codes (nibble i = column i) -> eight INT8 values through the table of their (row, group): two byte permutes
+// pick among entries 0..7 and 8..15 by the low three bits of each code, a third takes the right one by the code's top bit.
+__device__ __forceinline__ void expand8(std::uint32_t w, const uint4& t, std::uint32_t& lo, std::uint32_t& hi) {
+  const std::uint32_t s1 = w & 0x77777777u, s2 = ((w >> 1) & 0x44444444u) | 0x32103210u;
+  lo = __byte_perm(__byte_perm(t.x, t.y, s1), __byte_perm(t.z, t.w, s1), s2);
+  hi = __byte_perm(__byte_perm(t.x, t.y, s1 >> 16), __byte_perm(t.z, t.w, s1 >> 16), s2 >> 16);
+}
+
 // Programmatic dependent launch (see LaunchChain): both are no-ops in a kernel launched the ordinary way. A kernel may be
 // resident while kernels before it in its chain still write, and the wait orders ordinary loads only: what a kernel of the
 // same chain may write is never read with __ldg or any other read-only-cache load, which is for data that is constant

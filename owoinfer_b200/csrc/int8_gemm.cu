@@ -185,23 +185,6 @@ struct Shape {
 __host__ __device__ constexpr int out_warps(Epi e, int bn, bool w4) { return e == Epi::kAcc ? 0 : epi_warps(e, bn, w4); }
 __host__ __device__ constexpr int out_warp_bytes(Epi e) { return e == Epi::kSituGlu ? kSituOutWarpBytes : kOutWarpBytes; }
 
-// Eight 4-bit codes (nibble i = column i) -> eight INT8 values through the 16-entry table `t` of their (row, group):
-// two byte permutes pick among entries 0..7 and 8..15 by the low three bits of each code, a third takes the right one by
-// the code's top bit.
-__device__ __forceinline__ void expand8(std::uint32_t w, const uint4& t, std::uint32_t& lo, std::uint32_t& hi) {
-  const std::uint32_t s1 = w & 0x77777777u, s2 = ((w >> 1) & 0x44444444u) | 0x32103210u;
-  lo = __byte_perm(__byte_perm(t.x, t.y, s1), __byte_perm(t.z, t.w, s1), s2);
-  hi = __byte_perm(__byte_perm(t.x, t.y, s1 >> 16), __byte_perm(t.z, t.w, s1 >> 16), s2 >> 16);
-}
-__device__ __forceinline__ float e4m3_value(std::uint32_t b) {
-  const std::uint32_t e = (b >> 3) & 0xF, mant = b & 7;
-  float mag;
-  if (e == 0xF && mant == 7) mag = __int_as_float(0x7FC00000);
-  else if (e == 0) mag = static_cast<float>(mant) * 0.001953125f;  // 2^-9
-  else mag = __uint_as_float(((e + 120u) << 23) | (mant << 20));
-  return (b & 0x80) ? -mag : mag;
-}
-
 template <int kBN, Epi kEpi, int kCtas, bool kW4 = false>
 __global__ void __launch_bounds__(threads_of(kEpi, kBN, kW4), 1)
 int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
@@ -262,15 +245,9 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
   if constexpr (kW4) {
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-      const float sc = e4m3_value(static_cast<std::uint32_t>(i));
-      const bool ok = !(isnan(sc) || sc < 0.0f);
-      std::uint32_t wds[4] = {0u, 0u, 0u, 0u};
-      for (int c = 0; c < 16 && ok; ++c) {
-        const float level = p.w4_codebook != nullptr ? p.w4_codebook[c] : static_cast<float>(c) - 8.0f;
-        const float v = fminf(127.f, fmaxf(-127.f, rintf(fmul(level, sc))));
-        wds[c >> 2] |= (static_cast<std::uint32_t>(static_cast<int>(v)) & 0xFFu) << (8 * (c & 3));
-      }
-      s_lut[i] = make_uint4(wds[0], wds[1], wds[2], wds[3]);
+      s_lut[i] = w4_table(e4m3_value(static_cast<std::uint32_t>(i)), [&](int c) {
+        return p.w4_codebook != nullptr ? p.w4_codebook[c] : static_cast<float>(c) - 8.0f;
+      });
     }
   }
   if constexpr (kEpi == Epi::kSituGlu) {
@@ -1103,16 +1080,6 @@ int check_situ(const char* op, const b2_int8_operands* a, const void* out, std::
   }
   return B2_OK;
 }
-
-}  // namespace
-}  // namespace b2
-
-extern "C" {
-
-}  // extern "C"
-
-namespace b2 {
-namespace {
 
 int gemm_plain(const b2_int8_operands* op_, const void* bias, void* out, int64_t ldo, void* stream, int tile, bool early_weight) {
   constexpr const char* op = "int8_gemm";

@@ -625,23 +625,8 @@ __global__ void __launch_bounds__(256) unpack_int4_kernel(const std::uint8_t* pa
   }
 }
 
-__device__ __forceinline__ float e4m3_bits_to_float(std::uint32_t b) {
-  const std::uint32_t e = (b >> 3) & 0xF, mant = b & 7;
-  float mag;
-  if (e == 0xF && mant == 7) mag = __int_as_float(0x7FC00000);
-  else if (e == 0) mag = static_cast<float>(mant) * 0.001953125f;  // 2^-9
-  else mag = __uint_as_float(((e + 120u) << 23) | (mant << 20));
-  return (b & 0x80) ? -mag : mag;
-}
-
 // Raised (OR 1) by a decode that met a NaN or negative group scale and was given no word of the caller's.
 __device__ unsigned g_w4_invalid = 0;
-
-// Four 4-bit codes -> the bytes of the 16-entry table `t` (entry i in byte i % 4 of word i / 4): two byte permutes pick among
-// entries 0..7 and 8..15 by the low three bits of each code (s1), a third takes the right one by the code's top bit (s2).
-__device__ __forceinline__ u32 expand4(u32 s1, u32 s2, const uint4& t) {
-  return __byte_perm(__byte_perm(t.x, t.y, s1), __byte_perm(t.z, t.w, s1), s2);
-}
 
 constexpr int kDecodeUnroll = 4;
 
@@ -650,7 +635,8 @@ constexpr int kDecodeUnroll = 4;
 // whole groups, so everything is indexed by the flat column index; `shift` is log2(group), or -1 for other group sizes.
 // kTable (e4m3 scales): the 16 decoded values of every scale byte are tabulated once per block in shared memory, and a
 // thread expands its codes with byte permutes. Computing each value from its code and the row arithmetic (64-bit
-// divisions) held the kernel at 2.2 TB/s (56 us for a 24576 x 3072 weight); what bounds it now is HBM.
+// divisions) held the kernel at 2.0 TB/s (56 us for a 24576 x 3072 weight); it now takes 28.6 us (4.0 TB/s,
+// one launch after an L2 flush), bound by HBM.
 template <bool kTable>
 __global__ void __launch_bounds__(256) decode_grouped_kernel(const std::uint8_t* packed, const void* s_rel, const float* codebook,
                                                              std::int64_t items, int group, int shift, std::int8_t* out,
@@ -661,17 +647,8 @@ __global__ void __launch_bounds__(256) decode_grouped_kernel(const std::uint8_t*
   __shared__ uint4 s_table[kTable ? 256 : 1];
   if (threadIdx.x < 16) s_cb[threadIdx.x] = codebook != nullptr ? codebook[threadIdx.x] : static_cast<float>(threadIdx.x) - 8.0f;
   __syncthreads();
-  const auto decoded = [&](u32 code, float s) {
-    return static_cast<u32>(static_cast<int>(fminf(127.f, fmaxf(-127.f, rintf(fmul(s_cb[code], s)))))) & 0xFFu;
-  };
   if constexpr (kTable) {
-    const float s = e4m3_bits_to_float(threadIdx.x);
-    u32 t[4] = {0u, 0u, 0u, 0u};
-    if (!(isnan(s) || s < 0.0f)) {
-#pragma unroll
-      for (u32 c = 0; c < 16; ++c) t[c >> 2] |= decoded(c, s) << (8 * (c & 3));
-    }
-    s_table[threadIdx.x] = make_uint4(t[0], t[1], t[2], t[3]);
+    s_table[threadIdx.x] = w4_table(e4m3_value(threadIdx.x), [&](int c) { return s_cb[c]; });
     __syncthreads();
   }
   const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
@@ -700,11 +677,7 @@ __global__ void __launch_bounds__(256) decode_grouped_kernel(const std::uint8_t*
         bad |= (sb[u] & 0x7Fu) == 0x7Fu || sb[u] > 0x80u;  // NaN, or the sign bit over a non-zero magnitude
         const uint4 t = s_table[sb[u]];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const u32 s1 = w[j] & 0x77777777u, s2 = ((w[j] >> 1) & 0x44444444u) | 0x32103210u;
-          o[2 * j] = expand4(s1, s2, t);
-          o[2 * j + 1] = expand4(s1 >> 16, s2 >> 16, t);
-        }
+        for (int j = 0; j < 2; ++j) expand8(w[j], t, o[2 * j], o[2 * j + 1]);
       } else {
         const float s = __half2float(__ushort_as_half(static_cast<unsigned short>(sb[u])));
         const bool ok = !(isnan(s) || s < 0.0f);
@@ -713,7 +686,7 @@ __global__ void __launch_bounds__(256) decode_grouped_kernel(const std::uint8_t*
         for (int j = 0; j < 4; ++j) {
           u32 word = 0;
 #pragma unroll
-          for (int b = 0; b < 4; ++b) word |= decoded((w[j >> 1] >> (16 * (j & 1) + 4 * b)) & 0xFu, s) << (8 * b);
+          for (int b = 0; b < 4; ++b) word |= w4_byte(s_cb[(w[j >> 1] >> (16 * (j & 1) + 4 * b)) & 0xFu], s) << (8 * b);
           o[j] = ok ? word : 0u;
         }
       }
