@@ -318,23 +318,28 @@ typedef struct b2_block_run {
   int max_seqlen;
   int tier;                  /* B2_TIER_* */
   b2_attention_options attention;
-  int fused_norm_rope;       /* -1 auto (in the pre-pass whenever the run has no slots or tap; same bits either way, and
-                              * faster here at every size: the reference's 3072-row switch, dit_block_quant.cpp:32-35, is an
-                              * sm_89 measurement), 0 separate kernel, 1 in the pre-pass */
+  int fused_norm_rope;       /* -1 auto and 1: QK-norm + RoPE in the attention pre-pass, also with slots or a tap as long as
+                              * their rows are read and written in place (see slot_kv); 0: always their own kernel. Same
+                              * bits either way; the pre-pass is the faster at every size here (the reference's 3072-row
+                              * switch, dit_block_quant.cpp:32-35, is an sm_89 measurement) */
   /* Reference keys and reference prefill (BlockRun of src/models/moss_dit/dit_block_fused.h:132-147). A caller built
    * against a header that ends at fused_norm_rope passes that struct_size and gets none of it. All zero / NULL: unused.
    * slot_rows > 0: attention reads keys and values from the region [slot A | the run's tokens | slot B], slot_rows rows
    * per slot; sequence i's keys are rows [k0 + cu_seqlens_k[i], k0 + cu_seqlens_k[i + 1]) of it, k0 <= k1 bound the rows
    * the run reads, and max_seqlen covers the key lengths. slot_kv[s]: bf16 [slot_rows, 2 D], k | v per token as
-   * kv_tap wrote them (after QK-norm and RoPE), copied into slot s before attention; NULL for a slot the run does not
-   * read. QK-norm + RoPE then run as their own kernel on the run's own rows. */
+   * kv_tap wrote them (after QK-norm and RoPE); NULL for a slot the run does not read. The slot rows are read where they
+   * lie when every slot_kv that is read is 16-byte aligned, slot_kv_ld is a multiple of 8 and [k0, k1) holds all of the
+   * run's own rows; otherwise the block first copies them next to its own rows and QK-norm + RoPE run as their own kernel
+   * (same bits, slower: at 8484 own and 4096 slot rows 107 us of copies in a 2095 us block). */
   int64_t slot_rows;
   const void* slot_kv[2];
   int64_t slot_kv_ld;          /* elements between rows of slot_kv; 0 = 2 D (contiguous, as kv_tap writes them) */
   const int32_t* cu_seqlens_k; /* device int32 [batch + 1] */
   int64_t k0, k1;
   /* kv_tap != NULL: after QK-norm and RoPE the run's k and v rows are copied there as bf16 [tokens, 2 D]
-   * (tap_reference_kv, dit_block_fused.h:158); tap_only != 0: the block ends there, x untouched. */
+   * (tap_reference_kv, dit_block_fused.h:158): all of them, also rows that no sequence of cu_seqlens holds. Without slots
+   * and with a 16-byte aligned kv_tap the copy leaves with the pass that quantises the rows, otherwise it is one of its own.
+   * tap_only != 0: the block ends there, x untouched. */
   void* kv_tap;
   int tap_only;
 } b2_block_run;
@@ -578,7 +583,9 @@ int b2_dit_forward_graphed(b2_dit_graphs* graphs, const b2_dit_model* model, con
  * grids in heights / widths) run through every block as one sequence without text, under the modulation of
  * time_vector (the time vector of timestep 0 there), each with its reference RoPE table; block b's k | v rows after
  * QK-norm and RoPE land in kv_out[b] (device bf16 [num_blocks, sum h_i w_i, 2 D]). With the model's input extension
- * the extra channels are zero. workspace: b2_dit_prefill_workspace_bytes(). */
+ * the extra channels are zero. workspace: b2_dit_prefill_workspace_bytes(). The last block ends at its tap: its o,
+ * up_gate and down linears are checked like every other block's but not run, so a bad group scale among them reaches
+ * b2_w4_invalid_scales with the first forward. */
 typedef struct b2_prefill {
   size_t struct_size;
   const float* const* latents; /* host array of num_refs device pointers */

@@ -41,7 +41,7 @@ inline bool b200_can_run(const BlockTensors& w, const QuantBlockBuffers& a, cons
 
 // The b2_block_run of a run of the reference: D and F from the weights' shapes, heads = D / 128. With reference slots the
 // cached k | v rows are read where MossDit::forward put them, in the k | v columns of the slot rows of `big` (slot A
-// before all tokens, slot B after them: dit_block_fused.h:136-141); this library copies them next to its own QKV rows.
+// before all tokens, slot B after them: dit_block_fused.h:136-141).
 inline b2_block_run b200_block_run(const BlockTensors& w, const BlockRun& run, const QuantBlockBuffers* a = nullptr) {
   b2_block_run br{};
   br.struct_size = sizeof(b2_block_run);

@@ -39,8 +39,9 @@ int gemm_debug_set(unsigned long long wait_limit_ns, int skip_stage);
 // ---------------------------------------------------------------------------------------------------------------
 // Host: launches that overlap their predecessor's tail (programmatic dependent launch). While a LaunchChain is alive on
 // this thread, every kernel that enqueue() puts on its stream after the chain's first one may become resident as soon as
-// all blocks of the kernel before it have started; the kernels call dependents_may_start() first thing and
-// wait_for_predecessors() before they touch memory that anything on the stream may still be writing or reading. The
+// all blocks of the kernel before it have said so by dependents_may_start(), or have ended; the memory-bound kernels call
+// it first thing, the tensor-core ones when their last load is issued and up to kHandOverRows rows only. Every kernel calls
+// wait_for_predecessors() before it touches memory that anything on the stream may still be writing or reading. The
 // chain's first launch is an ordinary one, so whatever a caller enqueued before a call of this library is finished before
 // the call's first kernel starts: data that no kernel of the call writes may be read ahead of the wait.
 // At 2 x 320 tokens a launch takes the GPU about 2 us from the end of one kernel to the first instructions of the next
