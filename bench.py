@@ -219,8 +219,8 @@ def reference_kernels_on_this_gpu(torch, ops, keep, x, x0, mod, rope, cu, seq_le
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum, MB) of the four GEMM launches of one block at 16384 tokens,
 # F = 12288, from one ncu capture of exactly those launches. They describe the GEMM kernel as of GEMM_DRAM_COMMIT; a change
 # to its tile order or tile shape needs a new capture.
-GEMM_DRAM_MB = {"qkv": 83.3 + 255.0, "o": 160.6 + 54.2, "up_gate": 204.0 + 363.1, "down": 606.3 + 86.9}
-GEMM_DRAM_COMMIT = "7f7af74"
+GEMM_DRAM_MB = {"qkv": 82.3 + 255.2, "o": 160.6 + 54.3, "up_gate": 203.7 + 364.2, "down": 610.7 + 87.1}
+GEMM_DRAM_COMMIT = "bd30ba9"
 
 
 def gemm_sites(L, F):
@@ -527,9 +527,11 @@ def main():
     ws = torch.empty(ops.block_quant_workspace_bytes(run), dtype=torch.uint8, device="cuda")
     x = x0.clone()
     bufs = ops.block_buffers(x, mod, rope, ws)
-    launches_per_block = 12  # the grouped 4-bit tier decodes inside its GEMMs (e4m3 group scales): the same twelve launches
+    # Four quantisers, four GEMMs, four pre-pass launches, attention; the grouped 4-bit tier decodes each weight ahead of its
+    # GEMM at these row counts.
+    launches_per_block = 17 if tier == ops.TIER_W4A8 else 13
 
-    # The step (504 launches) is captured once into a CUDA graph and replayed, as the reference's engine does with its step
+    # The step (546 launches) is captured once into a CUDA graph and replayed, as the reference's engine does with its step
     # graphs; the first SiTU-GLU call fills its tables outside any capture, hence the eager call first.
     graph = None
     if not args.no_graph:

@@ -340,8 +340,8 @@ int b2_run_block_quant_sp(const b2_block_weights* w, const b2_block_buffers* a, 
     if (const int rc = cuda_ok(cudaEventRecord(comm->arrived[h], side))) return rc;
   }
 
-  // Attention over the full sequences, this rank's heads, half by half; QK-norm + RoPE in its pre-pass from 3072 tokens
-  // on. The return exchange of a half starts as soon as its attention is done.
+  // Attention over the full sequences, this rank's heads, half by half; QK-norm + RoPE in its pre-pass. The return
+  // exchange of a half starts as soon as its attention is done.
   const bool fused = r.fused_norm_rope != 0;  // automatic (< 0) = in the pre-pass, as in the single-GPU block
   const b2_qk_norm_rope nr{w->q_norm, w->k_norm, a->rope, 128};
   b2_attention_options ao = r.attention;

@@ -239,7 +239,7 @@ def measure_ulysses(rank: int, world: int, blocks: int, F: int, steps: int, warm
     rec = {"layout": f"{n_groups} group(s) x sequence-parallel {sp}", "groups": n_groups, "sp": sp, "sequences": seq_lens,
            "blocks": blocks, "ffn": F, "all_to_all_bytes_sent_per_gpu_per_block": sent, "kernel_status": list(ops.kernel_status()),
            "ms_with_local_copies_for_exchanges": ms_local, "exposed_exchange_ms": None if ms_local is None else ms - ms_local,
-           "launches_per_block": 16 + (2 * (sp - 1) * per_group * 2 if sp > 1 else 0)}
+           "launches_per_block": 19 + (2 * (sp - 1) * per_group * 2 if sp > 1 else 0)}
     comm.close()
     del weights, keep, blk, bufs
     torch.cuda.empty_cache()
