@@ -15,8 +15,8 @@ from . import _lib, build
 TRACE_LIB = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libowoinfer_b200_trace.so")
 
 # (stamp slot, what has just happened) in program order of a softmax warp's iteration u.
-SOFTMAX = [(4, "loop top"), (8, "scale of the sub-tile ready"), (0, "S(u) in registers (tcgen05.wait::ld)"), (1, "pass done: P(u) stored"),
-           (9, "vote: nothing to rescale"), (2, "denominator added"), (10, "fence.proxy.async"), (11, "tcgen05 fence + __syncwarp"),
+SOFTMAX = [(4, "loop top"), (8, "scale of the sub-tile ready"), (0, "S(u) in registers (tcgen05.wait::ld)"), (1, "pass done"),
+           (9, "vote: nothing to rescale"), (2, "pass stands"), (10, "P(u) in tensor memory"), (11, "tcgen05 fence + __syncwarp"),
            (3, "arrived on p_full(u)"), (12, "S(u+1) computed, P.V(u-1) landed (s_step wait)"), (13, "loads of S(u+1) issued"),
            (14, "headroom check done")]
 MMA = [(5, "p_full(u) seen"), (6, "P.V(u) issued"), (7, "Q.K^T(u+2) issued, step committed")]

@@ -12,7 +12,7 @@
 //     softmax         4 warps, one thread per query row: S -> fp32 (exact: |S| < 2^22), scaled by
 //                     sm_scale * log2e * q_scale * k_scale[64-key block], P = exp2(.) against a reference maximum that
 //                     is raised only when its headroom runs out (which makes rescaling O rare), denominator in fp32
-//                     from the unrounded P, P rounded to e4m3 into a swizzled shared tile
+//                     from the unrounded P, P rounded to e4m3 into tensor memory, over the scores it came from
 //     O += P8 · V8    tcgen05.mma kind::f8f6f4, fp32 accumulator in TMEM; V is read in its natural [key, channel]
 //                     layout as an MN-major operand, so the pre-pass needs no transpose
 //     out = O / d * v_scale[channel] -> bf16
@@ -676,41 +676,6 @@ __global__ void __launch_bounds__(256) quant_kv_kernel(const PrepArgs p) {
 #endif
 constexpr std::uint32_t kScoreBits = 0x4B400000u;                       // 12582912.0f
 constexpr std::uint32_t kScoreBias = B2_ATTN_CONST_BIAS ? 0u : kScoreBits;  // what a thread still has to add
-// Of every 8 scores (4 pairs) this many pairs take 2^x from a polynomial on the FMA pipe instead of the special-function
-// unit (0 = none).
-#ifndef B2_ATTN_POLY_PAIRS
-#define B2_ATTN_POLY_PAIRS 0
-#endif
-
-__device__ __forceinline__ std::uint64_t add2_rm(std::uint64_t a, std::uint64_t b) {
-  std::uint64_t d;
-  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ std::uint64_t sub2(std::uint64_t a, std::uint64_t b) {
-  std::uint64_t d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-// 2^x for a pair without the special-function unit: x = floor(x) + r by a round-down add of 1.5 * 2^23 (whose low
-// mantissa bits then hold floor(x)), a cubic for 2^r on [0, 1) (relative error below 1e-4, far inside the e4m3 rounding
-// of P), and the integer part added into the exponent field. Inputs below -125 give the result for -125 (< 2^-124: zero
-// for every use here).
-__device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float& p1) {
-  const std::uint64_t magic = pack2(12582912.f, 12582912.f);
-  const std::uint64_t x = pack2(fmaxf(x0, -125.f), fmaxf(x1, -125.f));
-  const std::uint64_t fl_m = add2_rm(x, magic);
-  const std::uint64_t r = sub2(x, sub2(fl_m, magic));
-  std::uint64_t p = fma2(pack2(0.0555054f, 0.0555054f), r, pack2(0.2402265f, 0.2402265f));
-  p = fma2(p, r, pack2(0.6931472f, 0.6931472f));
-  p = fma2(p, r, pack2(1.f, 1.f));
-  float q0, q1, f0, f1;
-  unpack2(p, q0, q1);
-  unpack2(fl_m, f0, f1);
-  p0 = __int_as_float(__float_as_int(q0) + (__float_as_int(f0) << 23));
-  p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(f1) << 23));
-}
-
 // One thread's 64 scores of a sub-tile, as read from tensor memory (four 16-column loads).
 struct ScoreRegs {
   std::uint32_t a[16], b[16], c[16], d[16];
@@ -723,28 +688,23 @@ __device__ __forceinline__ void load_scores(std::uint32_t s_cols, ScoreRegs& r) 
 }
 
 // One softmax pass of one thread over its row's 64 scores of a sub-tile, already in registers. P = exp2(f * c + bias)
-// with packed fp32 pairs for the FMA and the denominator (f the biased score, the constant folded into `bias`); e4m3 P goes
-// into the swizzled P tile (row = 128 bytes, 16-byte chunk n of row r stored at chunk n ^ (r % 8); this sub-tile owns
-// chunks chunk0 .. chunk0 + 3). Returns the largest biased score (0 if none) and the sum of the unrounded P.
+// with packed fp32 pairs for the FMA and the denominator (f the biased score, the constant folded into `bias`); e4m3 P comes
+// back packed, four keys to a word. Also returns the largest biased score (0 if none) and the sum of the unrounded P.
 template <bool kFull>
-__device__ __forceinline__ void softmax_pass(const ScoreRegs& s, float c, float bias, int valid, std::uint8_t* prow,
-                                             int chunk0, int row_xor, float& bmax_out, float& sum_out) {
+__device__ __forceinline__ void softmax_pass(const ScoreRegs& s, float c, float bias, int valid, std::uint32_t (&p)[16],
+                                             float& bmax_out, float& sum_out) {
   const std::uint64_t c2 = pack2(c, c), bias2 = pack2(bias, bias);
   std::uint64_t dA = pack2(0.f, 0.f), dB = dA;
   float bmax = 0.f;
-  const auto chunk = [&](const std::uint32_t (&r)[16], int n) {  // keys 16 n .. 16 n + 15 = one 16-byte chunk of the P row
+  const auto chunk = [&](const std::uint32_t (&r)[16], int n) {  // keys 16 n .. 16 n + 15
     float pv[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
       const float f0 = __uint_as_float(r[i] + kScoreBias), f1 = __uint_as_float(r[i + 1] + kScoreBias);
       float e0, e1;
       unpack2(fma2(pack2(f0, f1), c2, bias2), e0, e1);
-      if (((i >> 1) & 3) < B2_ATTN_POLY_PAIRS) {
-        exp2_poly2(e0, e1, pv[i], pv[i + 1]);
-      } else {
-        pv[i] = ex2(e0);
-        pv[i + 1] = ex2(e1);
-      }
+      pv[i] = ex2(e0);
+      pv[i + 1] = ex2(e1);
       if constexpr (kFull) {
         bmax = fmax3(bmax, f0, f1);
       } else {
@@ -759,9 +719,8 @@ __device__ __forceinline__ void softmax_pass(const ScoreRegs& s, float c, float 
       dA = add2(dA, pack2(pv[i], pv[i + 1]));
       dB = add2(dB, pack2(pv[i + 2], pv[i + 3]));
     }
-    *reinterpret_cast<uint4*>(prow + ((chunk0 + n) ^ row_xor) * 16) =
-        make_uint4(e4m3x4(pv[0], pv[1], pv[2], pv[3]), e4m3x4(pv[4], pv[5], pv[6], pv[7]),
-                   e4m3x4(pv[8], pv[9], pv[10], pv[11]), e4m3x4(pv[12], pv[13], pv[14], pv[15]));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) p[4 * n + i] = e4m3x4(pv[4 * i], pv[4 * i + 1], pv[4 * i + 2], pv[4 * i + 3]);
   };
   chunk(s.a, 0);
   chunk(s.b, 1);
@@ -791,9 +750,9 @@ constexpr int kTileQ = 128, kTileK = 128, kSubK = 64;
 constexpr int kKvStages = 2;
 constexpr int kTileBytes = 128 * 128;
 constexpr int kConstBytes = B2_ATTN_CONST_BIAS ? 128 * 32 : 0;  // the constant operand of the score bias: 128 rows of 16 bf16
-constexpr int kAttnSmem = kTileBytes * (1 + 2 * kKvStages + 1) + kConstBytes + 1024;  // Q, K/V stages, P, constant, alignment slack
+constexpr int kAttnSmem = kTileBytes * (1 + 2 * kKvStages) + kConstBytes + 1024;  // Q, K/V stages, constant, alignment slack
 constexpr int kAttnThreads = 192;  // TMA warp, MMA warp, 4 softmax warps
-constexpr std::uint32_t kTmemCols = 256;  // S(u % 2): columns [64 (u % 2), +64); O: columns [128, 256)
+constexpr std::uint32_t kTmemCols = 256;  // S(u % 2): columns [64 (u % 2), +64), P(u) in the first 16 of them; O: columns [128, 256)
 // Softmax reference maximum: set kHeadroom binades above what the largest P needs, raised again once fewer than kRaise
 // binades are left. e4m3 keeps full relative precision over 14 binades below p_range, so three binades of headroom cost
 // nothing measurable.
@@ -849,8 +808,12 @@ __device__ __forceinline__ void umma_bf16(std::uint32_t d_tmem, std::uint64_t a_
 //                 loop is a chain of latencies (barrier test, tensor-memory load, votes, fences), so it is software
 //                 pipelined: the loads of S(u + 1) are issued right after P(u) is handed over and land during the
 //                 bookkeeping in between, and the K scale of the next sub-tile is fetched a whole pass ahead.
-//   P             e4m3, the two buffers interleaved in one swizzled [128 x 128 B] tile: buffer i = bytes [64 i, +64) of
-//                 each row
+//   P             e4m3, the A operand of P·V in tensor memory (64 keys = 16 columns), in the first columns of the score
+//                 buffer it came from: the next scores go there by MMAs issued behind the ones that read P. With P in shared
+//                 memory (a swizzled 16 KB tile) one pair of sub-tiles kept the shared-memory port of an SM (128 bytes a
+//                 clock: the CTAs' K/V tiles in, the MMAs' operands out, P both ways) busy for about 1120 of the 1590 clocks
+//                 it took; without P it is 860. Kernel alone at 2 x 8192 tokens: 1212 -> 1166 us (1414 TOP/s), at 20480 keys
+//                 3649 -> 3516 us, at 4096 keys 194 -> 186 us; same bits.
 // kDump: the instantiation behind b2_attention_q8_debug_scores, which also stores one tile's raw integer scores.
 template <bool kDump>
 __global__ void __launch_bounds__(kAttnThreads, 2)
@@ -882,9 +845,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const std::uint32_t q_smem = base;
   const auto k_smem = [&](int s) { return base + kTileBytes * (1 + s); };
   const auto v_smem = [&](int s) { return base + kTileBytes * (1 + kKvStages + s); };
-  const std::uint32_t p_smem = base + kTileBytes * (1 + 2 * kKvStages);
-  const std::uint32_t const_smem = p_smem + kTileBytes;
-  std::uint8_t* p_generic = smem_raw + (p_smem - smem_u32(smem_raw));
+  const std::uint32_t const_smem = base + kTileBytes * (1 + 2 * kKvStages);
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&s_q_full), 1);
@@ -942,7 +903,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     constexpr std::uint32_t idesc_qk = umma_idesc(/*s32*/ 2, /*s8*/ 1, /*s8*/ 1, 0, 0, 128, kSubK);
     constexpr std::uint32_t idesc_pv = umma_idesc(/*f32*/ 1, /*e4m3*/ 0, /*e4m3*/ 0, 0, /*B MN-major*/ 1, 128, 128);
     constexpr std::uint32_t idesc_bias = umma_idesc(/*f32*/ 1, /*bf16*/ 1, /*bf16*/ 1, 0, 0, 128, kSubK);
-    const std::uint64_t dq = umma_desc_sw128(q_smem), dp = umma_desc_sw128(p_smem);
+    const std::uint64_t dq = umma_desc_sw128(q_smem);
     const std::uint64_t dconst = umma_desc_sw32(const_smem);
     static_assert(kKvStages == 2, "the descriptors below are selected, not indexed");
     const std::uint64_t dk0 = umma_desc_sw128(k_smem(0)), dk1 = umma_desc_sw128(k_smem(1));
@@ -998,10 +959,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (elect_one()) {
 #pragma unroll
         for (int k2 = 0; k2 < 2; ++k2) {
-          // P buffer u % 2: bytes [64 (u % 2), +64) of each row, 32 keys = 32 bytes along K inside the swizzle atom (+2);
-          // V (MN-major): 32 key rows of 128 bytes (+256 per step), second half of the tile at +kHalfTile.
-          umma_f8(tmem_o, dp + 2u * (2 * (u & 1) + k2), (s != 0 ? dv1 : dv0) + (u & 1) * kHalfTile + 256u * k2, idesc_pv,
-                  (u | k2) != 0 ? 1u : 0u);
+          // P(u): the first 16 columns of S(u), 32 keys to 8 columns; V (MN-major): 32 key rows of 128 bytes (+256 per
+          // step), second half of the tile at +kHalfTile.
+          umma_f8_ts(tmem_o, tmem_s + static_cast<std::uint32_t>(u & 1) * kSubK + 8u * k2,
+                     (s != 0 ? dv1 : dv0) + (u & 1) * kHalfTile + 256u * k2, idesc_pv, (u | k2) != 0 ? 1u : 0u);
         }
         if ((u & 1) != 0 || u + 1 >= n_sub) tc_commit(smem_u32(&s_v_empty[s]));
       }
@@ -1075,7 +1036,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&s_s_ready));
-    std::uint8_t* prow = p_generic + r_local * 128;
     bool dead = false;  // a bounded wait expired: leave without touching anything else
     ScoreRegs sr;
     float ks_cur = n_scales > 0 ? k_scale[0] : 0.f, ks_next = 0.f;
@@ -1086,8 +1046,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       load_scores(tmem_s + lane_off, sr);
     }
     for (int u = 0; !dead && u < n_sub; ++u) {
-      // Here S(u) is computed, P·V(u - 2) (which read this sub-tile's P buffer) has landed and the loads of S(u) are in
-      // flight.
+      // Here S(u) is computed, P·V(u - 2) has landed and the loads of S(u) are in flight.
       const std::uint32_t s_cols = tmem_s + lane_off + static_cast<std::uint32_t>(u & 1) * kSubK;
       TRACE(4);
       const float c = u < n_scales ? qs * ks_cur : 0.f;
@@ -1111,13 +1070,14 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (u == 0) m_run = (max_score(sr, valid) - 12582912.0f) * c - (a.p_offset - kHeadroom);
       bool o_idle = u < 1;  // every P·V up to u - 1 has to land before O is rescaled
       float mx, d_tile;
+      std::uint32_t p[16];  // P of this row, stored only once the pass stands: it takes the place of the scores
       for (;;) {
         const float bias = -fmaf(12582912.0f, c, m_run);
         float bmax;
         if (valid == kSubK) {
-          softmax_pass<true>(sr, c, bias, valid, prow, 4 * (u & 1), r_local & 7, bmax, d_tile);
+          softmax_pass<true>(sr, c, bias, valid, p, bmax, d_tile);
         } else {
-          softmax_pass<false>(sr, c, bias, valid, prow, 4 * (u & 1), r_local & 7, bmax, d_tile);
+          softmax_pass<false>(sr, c, bias, valid, p, bmax, d_tile);
         }
         TRACE(1);
         mx = bmax != 0.f ? (bmax - 12582912.0f) * c : kNone;
@@ -1149,11 +1109,12 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         tmem_ld_wait();
       }
       if (dead) break;
-      d_run += d_tile;
       TRACE(2);
-      // S is consumed and P written: both go to the MMA warp.
-      fence_proxy_async_smem();
+      tmem_st_32x16(s_cols, p);
+      d_run += d_tile;
+      tmem_st_wait();
       TRACE(10);
+      // S is consumed and P written: both go to the MMA warp.
       tc_fence_before();
       __syncwarp();
       TRACE(11);

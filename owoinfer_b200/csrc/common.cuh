@@ -317,13 +317,15 @@ __device__ __forceinline__ void umma_i8(std::uint32_t d_tmem, std::uint64_t a_de
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_f8(std::uint32_t d_tmem, std::uint64_t a_desc, std::uint64_t b_desc,
-                                        std::uint32_t idesc, std::uint32_t accumulate) {
+// The same with A in tensor memory: row r of A is lane r, four e4m3 values to a 32-bit column in K order (K = 32 is eight
+// columns from a_tmem on).
+__device__ __forceinline__ void umma_f8_ts(std::uint32_t d_tmem, std::uint32_t a_tmem, std::uint64_t b_desc,
+                                           std::uint32_t idesc, std::uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -425,6 +427,15 @@ __device__ __forceinline__ void tmem_st_32x32(std::uint32_t taddr, const std::ui
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
         "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
         "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
+      : "memory");
+}
+// The same for 16 consecutive columns.
+__device__ __forceinline__ void tmem_st_32x16(std::uint32_t taddr, const std::uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
 }
 // The same 32-bit value into this warp's 32 lanes x 32 consecutive columns.
