@@ -207,7 +207,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   constexpr int kEpiWarps = epi_warps(kEpi, kBN, kW4), kVecFloats = kEpi == Epi::kSituGlu ? 64 * (16 / epi_warps(kEpi, kBN, kW4)) : 384;
   __shared__ __align__(16) float s_vec[kEpiWarps][kVecFloats];
   // SiTU-GLU: the slices of the two factor tables, gate factors then hidden factors.
-  __shared__ std::uint16_t s_tab[kEpi == Epi::kSituGlu ? kMiniGate + kMiniHidden : 1];
+  __shared__ __align__(16) std::uint16_t s_tab[kEpi == Epi::kSituGlu ? kMiniGate + kMiniHidden : 1];
 
   const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
   const std::uint32_t tiles_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -248,24 +248,6 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       s_lut[i] = w4_table(e4m3_value(static_cast<std::uint32_t>(i)), [&](int c) {
         return p.w4_codebook != nullptr ? p.w4_codebook[c] : static_cast<float>(c) - 8.0f;
       });
-    }
-  }
-  if constexpr (kEpi == Epi::kSituGlu) {
-    const auto fill = [&](auto load) {
-      for (int i = threadIdx.x; i < kMiniGate + kMiniHidden; i += blockDim.x) {
-        const bool gate = i < kMiniGate;
-        const std::uint32_t j = gate ? i : i - kMiniGate;  // [sign (gate only)][exponent][mantissa]
-        const std::uint32_t bits = ((j >> 12) << 15) | ((((j >> 7) & 31u) + kMiniExpLo) << 7) | (j & 127u);
-        s_tab[i] = load((gate ? p.t_gate : p.t_hidden) + bits);
-      }
-    };
-    // Tables of an earlier call are constant: the read-only cache's loads run ahead of the shared stores. Tables that this
-    // very chain of launches fills are not.
-    if (p.early_tables != 0) {
-      fill([](const std::uint16_t* at) { return __ldg(at); });
-    } else {
-      wait_for_predecessors();
-      fill([](const std::uint16_t* at) { return *at; });
     }
   }
   tc_fence_before();
@@ -502,7 +484,26 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // Epilogue: 8 warps. Warp w may touch TMEM lanes [32 (w % 4), 32 (w % 4) + 32); warps 2..5 take the first half of the
     // tile's columns, warps 6..9 the second half (SiTU-GLU: output columns, each needing its hidden and gate accumulator).
     const int quarter = warp & 3, col_half = (warp - 2) >> 2;  // SiTU-GLU: one of four 32-column parts
-    wait_for_predecessors();
+    constexpr int kPart = kBN / (kEpiWarps / 4);  // the columns of the tile that this warp finishes: [part0, part0 + kPart)
+    const int part0 = col_half * kPart;
+    // Tables of an earlier call are constant: they are fetched ahead of the wait. Tables that this very chain of launches
+    // fills are not. Only the warps that look them up wait for the slices (three runs of 4096 entries, 16 bytes at a time);
+    // the first loads and MMAs go ahead meanwhile. (All threads fetching entry by entry ahead of the first load: 34.5 us
+    // instead of 31.4 at 297 rows, F = 12288; 46.4 instead of 43.4 at 586.)
+    if (kEpi != Epi::kSituGlu || p.early_tables == 0) wait_for_predecessors();
+    if constexpr (kEpi == Epi::kSituGlu) {
+      const int t = (warp - 2) * 32 + lane;
+#pragma unroll
+      for (int part = 0; part < 3; ++part) {  // gate, positive and negative; hidden, positive
+        const std::uint16_t* from = (part < 2 ? p.t_gate : p.t_hidden) + (part == 1 ? 0x8000u : 0u) + (kMiniExpLo << 7);
+        for (int i = t; i < kMiniHidden / 8; i += 32 * kEpiWarps) {
+          const uint4* at = reinterpret_cast<const uint4*>(from) + i;
+          reinterpret_cast<uint4*>(s_tab)[part * (kMiniHidden / 8) + i] = p.early_tables != 0 ? __ldg(at) : *at;
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+      if (p.early_tables != 0) wait_for_predecessors();
+    }
     std::uint32_t tile_it = 0;
     for (int tile = tile0; tile < total_tiles; tile += tile_step, ++tile_it) {
       int mt, nt;
@@ -513,7 +514,6 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       float* vec = s_vec[warp - 2];
       __syncwarp();
       if constexpr (kEpi != Epi::kAcc) {  // the accumulator dump reads no per-column vector (and allows any n)
-        constexpr int kHalfCols = kBN / (kEpiWarps / 4);  // columns of one warp's part of the tile
         // SiTU-GLU: a warp takes 32-column parts col_half, col_half + kEpiWarps / 4, ... of the tile's 128 output columns
         // (one part with 16 epilogue warps, two with 8); 64 floats per part.
         constexpr int kSituParts = kEpi == Epi::kSituGlu ? 16 / kEpiWarps : 1;
@@ -526,8 +526,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             col = ((j & 63) < 32 ? 0 : p.half) + oc;
             ok = oc < p.half;
           } else {
-            col = nt * kBN + col_half * kHalfCols + j;
-            ok = j < kHalfCols && col < p.n;
+            col = nt * kBN + part0 + j;
+            ok = j < kPart && col < p.n;
           }
           float4 w = make_float4(0.f, 0.f, 0.f, 0.f), b = w, g = w;
           if (ok) {
@@ -556,6 +556,19 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
       }
       __syncwarp();
+      // Gated residual: the residual rows of the warp's first 64 columns are asked for ahead of the accumulator (and those
+      // of the next 64 ahead of the work on these), so that their way from L2 is not part of a tile's last microseconds:
+      // 0.4 to 0.8 us of a launch from 297 to 1050 rows. (The W4A8 kernels have no registers left for it.)
+      [[maybe_unused]] uint4 ahead_res[8];
+      [[maybe_unused]] const auto fetch_residual = [&](int c0) {
+        const int pcol = nt * kBN + c0 + 8 * (lane & 7), r0 = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM + quarter * 32 + (lane >> 3);
+        if (pcol >= p.n) return;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (r0 + 4 * i < p.m) ahead_res[i] = *reinterpret_cast<const uint4*>(p.out + static_cast<std::int64_t>(r0 + 4 * i) * p.ldo + pcol);
+        }
+      };
+      if constexpr (kEpi == Epi::kGatedResidual && !kW4) fetch_residual(part0);
       if (!wait_bar(smem_u32(&s_tmem_full[acc]), acc_ph, abort_word)) break;
       tc_fence_after();
       const int row = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM + quarter * 32 + lane;
@@ -649,9 +662,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
       } else {
         const int col0 = nt * kBN;
-        constexpr int kHalfCols = kBN / (kEpiWarps / 4);
 #pragma unroll 1
-        for (int c0 = col_half * kHalfCols; c0 < (col_half + 1) * kHalfCols; c0 += 64) {
+        for (int c0 = part0; c0 < part0 + kPart; c0 += 64) {
           std::uint32_t r[64];
           tmem_ld_32x32(t_row + c0, *reinterpret_cast<std::uint32_t(*)[32]>(&r[0]));
           tmem_ld_32x32(t_row + c0 + 32, *reinterpret_cast<std::uint32_t(*)[32]>(&r[32]));
@@ -691,9 +703,12 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                   const int r = row_base + sub + 4 * i;
                   if (r < p.m) {
                     *reinterpret_cast<uint4*>(stage_tile + (sub + 4 * i) * kOutRowBytes + 16 * piece) =
-                        *reinterpret_cast<const uint4*>(global_piece(r));
+                        kW4 ? *reinterpret_cast<const uint4*>(global_piece(r)) : ahead_res[i];
                   }
                 }
+              }
+              if constexpr (!kW4) {
+                if (c0 + 64 < part0 + kPart) fetch_residual(c0 + 64);
               }
               __syncwarp();
             }
@@ -702,7 +717,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               for (int v = 0; v < 8; ++v) {
                 const int col = col0 + c0 + 8 * v;
                 if (col >= p.n) continue;  // n % 8 == 0: a vector of 8 columns is all in or all out
-                const int lc = c0 - col_half * kHalfCols + 8 * v;  // column inside this warp's half
+                const int lc = c0 - part0 + 8 * v;  // column inside this warp's part
                 const float4 w0 = *reinterpret_cast<const float4*>(vec + lc);
                 const float4 w1 = *reinterpret_cast<const float4*>(vec + lc + 4);
                 const float4 b0 = *reinterpret_cast<const float4*>(vec + 128 + lc);
@@ -774,8 +789,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // bf16(bf16(4 * bf16(tanh(bf16(x / 4)))) * bf16(sigmoid(x))) and hidden factor bf16(25 * bf16(tanh(bf16(x * fp32(1/25))))).
 // Reference: src/kernels/fused/fused_gemm_impl.cuh:58-67, src/kernels/quant/int8_gemm_situ.cu:16-27.
 // ---------------------------------------------------------------------------------------------------------------
-__device__ std::uint16_t g_situ_gate[65536];
-__device__ std::uint16_t g_situ_hidden[65536];
+__device__ __align__(16) std::uint16_t g_situ_gate[65536];
+__device__ __align__(16) std::uint16_t g_situ_hidden[65536];
 
 __global__ void fill_situ_tables() {
   const std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
