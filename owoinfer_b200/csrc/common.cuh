@@ -317,8 +317,8 @@ __device__ __forceinline__ void umma_i8(std::uint32_t d_tmem, std::uint64_t a_de
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The same with A in tensor memory: row r of A is lane r, four e4m3 values to a 32-bit column in K order (K = 32 is eight
-// columns from a_tmem on).
+// The same for e4m3 operands with A in tensor memory: row r of A is lane r, four values to a 32-bit column in K order (K = 32
+// is eight columns from a_tmem on).
 __device__ __forceinline__ void umma_f8_ts(std::uint32_t d_tmem, std::uint32_t a_tmem, std::uint64_t b_desc,
                                            std::uint32_t idesc, std::uint32_t accumulate) {
   asm volatile(
@@ -343,6 +343,10 @@ __device__ __forceinline__ std::uint32_t map_to_cta(std::uint32_t smem_addr, std
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes into the shared memory of a CTA of the cluster (shared::cluster address).
+__device__ __forceinline__ void st_cluster_v4(std::uint32_t cluster_addr, std::uint32_t x, std::uint32_t y, std::uint32_t z, std::uint32_t w) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 // Arrive on an mbarrier given by its shared::cluster address (own or peer CTA).
 __device__ __forceinline__ void mbar_arrive_cluster(std::uint32_t cluster_addr) {

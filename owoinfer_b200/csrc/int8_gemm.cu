@@ -185,15 +185,23 @@ struct Shape {
 __host__ __device__ constexpr int out_warps(Epi e, int bn, bool w4) { return e == Epi::kAcc ? 0 : epi_warps(e, bn, w4); }
 __host__ __device__ constexpr int out_warp_bytes(Epi e) { return e == Epi::kSituGlu ? kSituOutWarpBytes : kOutWarpBytes; }
 
-template <int kBN, Epi kEpi, int kCtas, bool kW4 = false>
+// kSplit > 1: a cluster of kSplit such tiles' CTAs (pairs) works on ONE output tile, each on its part of K. When their MMAs
+// are done every CTA hands the others' columns of its int32 accumulator over through distributed shared memory (into the
+// ring, which is idle by then) and finishes its own kBN / kSplit columns: exact sums, so the same bits. For problems of so
+// few tiles that half of the SMs would idle; the sums through L2 instead had cost 8 to 17 us a launch, this costs 1 to 2.
+template <int kBN, Epi kEpi, int kCtas, bool kW4 = false, int kSplit = 1>
 __global__ void __launch_bounds__(threads_of(kEpi, kBN, kW4), 1)
 int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   static_assert(kCtas == 1 || kBN == 256, "CTA pairs run 256 x 256 tiles");
   static_assert(!kW4 || kBN / kCtas == 128, "W4A8: one weight row of the stage per converter thread");
+  static_assert(kSplit == 1 || (!kW4 && (kEpi == Epi::kPlain || kEpi == Epi::kGatedResidual) && kBN / kSplit >= 64), "split tiles");
   using S = Shape<kBN, kCtas, kW4, out_warps(kEpi, kBN, kW4), out_warp_bytes(kEpi)>;
-  const std::uint32_t rank = kCtas == 2 ? cluster_ctarank() : 0u;   // CTA of the pair; rank 0 issues the MMAs
-  const int tile0 = kCtas == 2 ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-  const int tile_step = kCtas == 2 ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+  constexpr int kCluster = kCtas * kSplit;
+  const std::uint32_t cta = kCluster > 1 ? cluster_ctarank() : 0u;
+  const std::uint32_t rank = cta & (kCtas - 1);  // CTA of the pair; rank 0 issues the MMAs
+  const std::uint32_t leader = cta - rank;       // that CTA in the cluster
+  const int split = static_cast<int>(cta) / kCtas;
+  const int tile0 = static_cast<int>(blockIdx.x) / kCluster, tile_step = static_cast<int>(gridDim.x) / kCluster;
   constexpr int kStages = S::kStages;
   extern __shared__ std::uint8_t smem_raw[];
   __shared__ __align__(8) std::uint64_t s_full[kStages], s_empty[kStages], s_tmem_full[2], s_tmem_empty[2];
@@ -252,12 +260,13 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (kCtas == 2) cluster_sync_all();  // the peer's barriers exist before anything arrives on them
+  if constexpr (kCluster > 1) cluster_sync_all();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const std::uint32_t tmem_base = s_tmem_base;
   volatile int* abort_word = &s_abort;
 
-  const int k_blocks = (p.k + kBK - 1) / kBK;
+  const int k_blocks_all = (p.k + kBK - 1) / kBK;
+  const int kb_first = k_blocks_all * split / kSplit, k_blocks = k_blocks_all * (split + 1) / kSplit;  // this CTA's K blocks
   const int total_tiles = p.m_tiles * p.n_tiles;
 
   if (warp == 0) {
@@ -281,13 +290,13 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           int mt, nt, row_b0, row_b1;
           tile_coords(p, tile0, &mt, &nt);
           b_rows(nt, row_b0, row_b1);
-          ahead = static_cast<std::uint32_t>(min(kStages, k_blocks));
+          ahead = static_cast<std::uint32_t>(min(kStages, k_blocks - kb_first));
           for (std::uint32_t s = 0; s < ahead; ++s) {
             const std::uint32_t full = smem_u32(&s_full[s]);
-            const int c0 = static_cast<int>(s) * kBK;
+            const int c0 = (kb_first + static_cast<int>(s)) * kBK;
             if constexpr (kCtas == 2) {
               if (rank == 0) mbar_expect_tx(full, 2 * S::kStageBytes);
-              tma_load_2d_pair(b_addr(s), &map_b, map_to_cta(full, 0), c0, row_b0);
+              tma_load_2d_pair(b_addr(s), &map_b, map_to_cta(full, leader), c0, row_b0);
             } else {
               mbar_expect_tx(full, S::kStageBytes);
               tma_load_2d(b_addr(s), &map_b, full, c0, row_b0);
@@ -304,7 +313,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         int row_b0, row_b1;
         b_rows(nt, row_b0, row_b1);
         const bool skip_last = g_gemm_test_skip_stage != 0 && tile == tile0;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        for (int kb = kb_first; kb < k_blocks; ++kb, ++it) {
           const int s = static_cast<int>(it % kStages);
           const std::uint32_t ph = (it / kStages) & 1u;
           if (!wait_bar(smem_u32(&s_empty[s]), ph ^ 1u, abort_word)) break;
@@ -315,7 +324,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             // barrier, where its converter warps pick it up.
             if constexpr (kCtas == 2) {
               if (rank == 0) mbar_expect_tx(full, 2 * S::kABytes);
-              tma_load_2d_pair(a_addr(s), &map_a, map_to_cta(full, 0), kb * kBK, row_a);
+              tma_load_2d_pair(a_addr(s), &map_a, map_to_cta(full, leader), kb * kBK, row_a);
             } else {
               mbar_expect_tx(full, S::kABytes);
               tma_load_2d(a_addr(s), &map_a, full, kb * kBK, row_a);
@@ -324,12 +333,12 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             mbar_expect_tx(pfull, S::kPBytes);
             tma_load_2d(p_addr(s), &map_b, pfull, kb * (kBK / 2), row_b0);
           } else if (it < ahead) {  // the weight tile is on its way already
-            if constexpr (kCtas == 2) tma_load_2d_pair(a_addr(s), &map_a, map_to_cta(full, 0), kb * kBK, row_a);
+            if constexpr (kCtas == 2) tma_load_2d_pair(a_addr(s), &map_a, map_to_cta(full, leader), kb * kBK, row_a);
             else tma_load_2d(a_addr(s), &map_a, full, kb * kBK, row_a);
           } else if constexpr (kCtas == 2) {
             // Both CTAs' copies complete on the leader's barrier, which expects the bytes of the whole pair.
             if (rank == 0) mbar_expect_tx(full, 2 * S::kStageBytes);
-            const std::uint32_t full_leader = map_to_cta(full, 0);
+            const std::uint32_t full_leader = map_to_cta(full, leader);
             tma_load_2d_pair(a_addr(s), &map_a, full_leader, kb * kBK, row_a);
             tma_load_2d_pair(b_addr(s), &map_b, full_leader, kb * kBK, row_b0);
           } else {
@@ -344,6 +353,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (p.hand_over != 0) dependents_may_start();
     }
     __syncwarp();
+    if constexpr (kSplit > 1) cluster_sync_all(), cluster_sync_all();  // (the epilogue warps' two)
   } else if (warp == 1) {
     // The whole warp of the issuing CTA walks the loop (uniform control flow, so descriptors and loop state stay in
     // uniform registers; every lane takes the waits); one elected lane issues the MMAs and commits.
@@ -361,7 +371,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (!ok) break;
         tc_fence_after();
         const std::uint32_t d_tmem = tmem_base + acc * kBN;
-        for (int kb = 0; kb < k_blocks; ++kb) {
+        for (int kb = kb_first; kb < k_blocks; ++kb) {
           ok = wait_bar(smem_u32(&s_full[s]), ph, abort_word);
           ok = !__any_sync(0xffffffffu, !ok);
           if (!ok) break;
@@ -373,13 +383,13 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               // 32 bytes further along K inside the swizzle atom: +2 in the descriptor's 16-byte address units.
               if constexpr (kCtas == 2) {
                 umma_i8_pair(d_tmem, da + static_cast<std::uint64_t>(2 * k4), db + static_cast<std::uint64_t>(2 * k4), idesc,
-                             (kb | k4) != 0 ? 1u : 0u);
+                             (kb != kb_first || k4 != 0) ? 1u : 0u);
               } else {
                 umma_i8(d_tmem, da + static_cast<std::uint64_t>(2 * k4), db + static_cast<std::uint64_t>(2 * k4), idesc,
-                        (kb | k4) != 0 ? 1u : 0u);
+                        (kb != kb_first || k4 != 0) ? 1u : 0u);
               }
             }
-            if constexpr (kCtas == 2) tc_commit_pair(smem_u32(&s_empty[s]), 3);
+            if constexpr (kCtas == 2) tc_commit_pair(smem_u32(&s_empty[s]), static_cast<std::uint16_t>(3u << leader));
             else tc_commit(smem_u32(&s_empty[s]));
           }
           __syncwarp();
@@ -387,13 +397,14 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
         if (!ok) break;
         if (elect_one()) {
-          if constexpr (kCtas == 2) tc_commit_pair(smem_u32(&s_tmem_full[acc]), 3);
+          if constexpr (kCtas == 2) tc_commit_pair(smem_u32(&s_tmem_full[acc]), static_cast<std::uint16_t>(3u << leader));
           else tc_commit(smem_u32(&s_tmem_full[acc]));
         }
         __syncwarp();
       }
     }
     __syncwarp();
+    if constexpr (kSplit > 1) cluster_sync_all(), cluster_sync_all();
   } else if (kW4 && warp >= 2 + kEpiWarps) {
     // W4A8 converters: two threads per weight row of the CTA's 128-row stage, 64 columns each. Per K block a thread reads
     // its 32 packed bytes (TMA wrote the tile with the 64-byte swizzle: 16-byte chunk c of row r sits at chunk
@@ -471,7 +482,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if constexpr (kCtas == 2) mbar_arrive_cluster(map_to_cta(smem_u32(&s_full[s]), 0));
+          if constexpr (kCtas == 2) mbar_arrive_cluster(map_to_cta(smem_u32(&s_full[s]), leader));
           else mbar_arrive(smem_u32(&s_full[s]));
         }
 #pragma unroll
@@ -484,8 +495,14 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // Epilogue: 8 warps. Warp w may touch TMEM lanes [32 (w % 4), 32 (w % 4) + 32); warps 2..5 take the first half of the
     // tile's columns, warps 6..9 the second half (SiTU-GLU: output columns, each needing its hidden and gate accumulator).
     const int quarter = warp & 3, col_half = (warp - 2) >> 2;  // SiTU-GLU: one of four 32-column parts
-    constexpr int kPart = kBN / (kEpiWarps / 4);  // the columns of the tile that this warp finishes: [part0, part0 + kPart)
-    const int part0 = col_half * kPart;
+    // The columns of the tile that this warp finishes: [part0, part0 + kPart). Split tiles: the tile's 64-column units belong
+    // to the splits in order, and a unit of a split to the warps of col_half = unit % 2 (a split that owns one unit leaves
+    // the other warps' part empty).
+    constexpr int kPart = kSplit > 1 ? 64 : kBN / (kEpiWarps / 4);
+    constexpr int kOwnUnits = kBN / 64 / kSplit;
+    const int own_unit = kSplit == 1 ? 0 : kOwnUnits == 2 ? split * 2 + col_half : split;
+    const bool has_part = kSplit == 1 || kOwnUnits == 2 || (own_unit & 1) == col_half;
+    const int part0 = kSplit > 1 ? own_unit * 64 : col_half * kPart;
     // Tables of an earlier call are constant: they are fetched ahead of the wait. Tables that this very chain of launches
     // fills are not. Only the warps that look them up wait for the slices (three runs of 4096 entries, 16 bytes at a time);
     // the first loads and MMAs go ahead meanwhile. (All threads fetching entry by entry ahead of the first load: 34.5 us
@@ -568,9 +585,40 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (r0 + 4 * i < p.m) ahead_res[i] = *reinterpret_cast<const uint4*>(p.out + static_cast<std::int64_t>(r0 + 4 * i) * p.ldo + pcol);
         }
       };
-      if constexpr (kEpi == Epi::kGatedResidual && !kW4) fetch_residual(part0);
-      if (!wait_bar(smem_u32(&s_tmem_full[acc]), acc_ph, abort_word)) break;
+      if constexpr (kEpi == Epi::kGatedResidual && !kW4) {
+        if (has_part) fetch_residual(part0);
+      }
+      bool landed = wait_bar(smem_u32(&s_tmem_full[acc]), acc_ph, abort_word);
+      if constexpr (kSplit == 1) {
+        if (!landed) break;
+      }
       tc_fence_after();
+      if constexpr (kSplit > 1) {
+        // Every CTA of the cluster is past its last MMA: the rings are free. Accumulator columns of the other splits go to
+        // their CTA of the same rows, 16 bytes per lane side by side, where the same lane of that CTA finds them.
+        landed = !__any_sync(0xffffffffu, !landed);
+        cluster_sync_all();
+        if (landed) {
+#pragma unroll 1
+          for (int unit = col_half; unit < kBN / 64; unit += 2) {
+            const int owner = unit / kOwnUnits;
+            if (owner == split) continue;
+            const int slot = split < owner ? split : split - 1;
+            const std::uint32_t at = map_to_cta(tiles_base, static_cast<std::uint32_t>(owner * kCtas) + rank) +
+                                     static_cast<std::uint32_t>(((slot * kOwnUnits + unit % kOwnUnits) * 4 + quarter) * 8192 + lane * 16);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              std::uint32_t v[32];
+              tmem_ld_32x32(tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + unit * 64 + 32 * h, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 8; ++i) st_cluster_v4(at + static_cast<std::uint32_t>(8 * h + i) * 512, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            }
+          }
+        }
+        cluster_sync_all();
+        if (!landed || !has_part) break;
+      }
       const int row = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM + quarter * 32 + lane;
       const bool row_ok = row < p.m;
       const float xs = row_ok ? p.xs[row] : 0.f;
@@ -668,6 +716,17 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           tmem_ld_32x32(t_row + c0, *reinterpret_cast<std::uint32_t(*)[32]>(&r[0]));
           tmem_ld_32x32(t_row + c0 + 32, *reinterpret_cast<std::uint32_t(*)[32]>(&r[32]));
           tmem_ld_wait();
+          if constexpr (kSplit > 1) {
+            const std::uint8_t* got = smem_raw + (tiles_base - smem_u32(smem_raw)) + ((own_unit % kOwnUnits) * 4 + quarter) * 8192 + lane * 16;
+#pragma unroll
+            for (int slot = 0; slot < kSplit - 1; ++slot) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const uint4 v = *reinterpret_cast<const uint4*>(got + slot * kOwnUnits * 4 * 8192 + i * 512);
+                r[4 * i] += v.x, r[4 * i + 1] += v.y, r[4 * i + 2] += v.z, r[4 * i + 3] += v.w;
+              }
+            }
+          }
           if constexpr (kEpi == Epi::kAcc) {
             if (!row_ok) continue;
             std::int32_t* arow = p.acc + static_cast<std::int64_t>(row) * p.ldacc;
@@ -761,7 +820,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        if constexpr (kCtas == 2) mbar_arrive_cluster(map_to_cta(smem_u32(&s_tmem_empty[acc]), 0));
+        if constexpr (kCtas == 2) mbar_arrive_cluster(map_to_cta(smem_u32(&s_tmem_empty[acc]), leader));
         else mbar_arrive(smem_u32(&s_tmem_empty[acc]));
       }
     }
@@ -776,7 +835,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
     __syncthreads();
   }
-  if constexpr (kCtas == 2) cluster_sync_all();  // nothing of the pair is in flight towards this CTA any more
+  if constexpr (kCluster > 1) cluster_sync_all();  // nothing of the cluster is in flight towards this CTA any more
   if (warp == 1) {
     tc_fence_after();
     if constexpr (kCtas == 2) tmem_dealloc_pair(tmem_base, 512);
@@ -899,7 +958,7 @@ int check_output(const char* op, const char* name, const void* p, std::int64_t l
 }
 
 // kW4: a->w points at the packed 4-bit codes [n, k / 2] (p.w4_* describe the rest of the weight).
-template <int kBN, Epi kEpi, int kCtas, bool kW4 = false>
+template <int kBN, Epi kEpi, int kCtas, bool kW4 = false, int kSplit = 1>
 int launch_kernel(const char* op, const b2_int8_operands* a, GemmParams p, cudaStream_t stream) {
   using S = Shape<kBN, kCtas, kW4, out_warps(kEpi, kBN, kW4), out_warp_bytes(kEpi)>;
   CUtensorMap map_a, map_b;
@@ -916,7 +975,7 @@ int launch_kernel(const char* op, const b2_int8_operands* a, GemmParams p, cudaS
                                  static_cast<std::uint64_t>(a->k), kBK, 128, op)) {
     return B2_ERR_CUDA;
   }
-  auto kernel = int8_gemm_kernel<kBN, kEpi, kCtas, kW4>;
+  auto kernel = int8_gemm_kernel<kBN, kEpi, kCtas, kW4, kSplit>;
   // Opt in to the large dynamic shared-memory size once per device and instantiation.
   // (Setting the attribute twice from two threads is harmless; the flag only saves the call.)
   static std::atomic<bool> configured[64] = {};
@@ -947,8 +1006,9 @@ int launch_kernel(const char* op, const b2_int8_operands* a, GemmParams p, cudaS
       p.band_m = std::max(p.band_m, static_cast<int>(resident));
     }
   }
-  const int grid = kCtas == 2 ? 2 * std::min(total, sm_count() / 2) : std::min(total, sm_count());
-  return enqueue(op, kernel, grid, threads_of(kEpi, kBN, kW4), S::kSmemBytes, stream, kCtas, map_a, map_b, p);
+  // (A split tile's cluster ends with its one tile.)
+  const int grid = kSplit > 1 ? total * kCtas * kSplit : kCtas == 2 ? 2 * std::min(total, sm_count() / 2) : std::min(total, sm_count());
+  return enqueue(op, kernel, grid, threads_of(kEpi, kBN, kW4), S::kSmemBytes, stream, kCtas * kSplit, map_a, map_b, p);
 }
 
 // Tile choice of the W4A8 GEMM: CTA pairs on 256 x 256 tiles when there are enough of them to fill the GPU; else one CTA
@@ -974,6 +1034,40 @@ int pick_tile(int tile, std::int64_t m, std::int64_t n_tiles_256) {
 struct TileCost {
   double fixed, per_block;
 };
+// Tiles whose K range a cluster shares (never asked for by a caller). Measured, 3072 columns, us (rows x K):
+//                128 x 128   pairs   128 x 128 in two   pairs in two   pairs in four
+//   100 x 12288    30.3      35.9         20.2              23.7           19.6
+//   297 x 3072     12.1      15.5         11.0              13.2
+//   297 x 8192     22.1      27.2         16.4              19.2
+//   400 x 8192     22.3      27.1                           19.5
+//   400 x 12288    30.7      36.3                           24.2
+constexpr int kTilePairs2 = 16, kTilePairs4 = 17, kTile128x2 = 18;
+// How many clusters of a split tile's kernel the device holds at once (asked once per device): a grid of more would run in
+// two rounds. (Clusters of four reach 132 of a B200's 148 SMs, of eight 120.)
+template <int kBN, Epi kEpi, int kCtas, int kSplit>
+int resident_clusters() {
+  using S = Shape<kBN, kCtas, false, out_warps(kEpi, kBN, false), out_warp_bytes(kEpi)>;
+  static std::atomic<int> cached[64] = {};  // clusters + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = cached[dev].load(std::memory_order_relaxed) - 1;
+  if (n < 0) {
+    const auto kernel = int8_gemm_kernel<kBN, kEpi, kCtas, false, kSplit>;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kCtas * kSplit, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
+    cfg.gridDim = kCtas * kSplit, cfg.blockDim = threads_of(kEpi, kBN, false), cfg.dynamicSmemBytes = S::kSmemBytes, cfg.attrs = &attr, cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    cached[dev].store(n + 1, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 template <Epi kEpi>
 int pick_tile_int8(const GemmParams& p) {
   constexpr bool kSitu = kEpi == Epi::kSituGlu;
@@ -986,7 +1080,20 @@ int pick_tile_int8(const GemmParams& p) {
   };
   const double pair = cost(kPair, (m_tiles + 1) / 2 * n256, sms / 2), big = cost(kBig, m_tiles * n256, sms);
   const double small = kSitu ? big : cost(kSmall, m_tiles * n128, sms);
-  return pair <= big && pair <= small ? B2_TILE_2CTA_256x256 : big <= small ? B2_TILE_128x256 : B2_TILE_128x128;
+  int best = pair <= big && pair <= small ? B2_TILE_2CTA_256x256 : big <= small ? B2_TILE_128x256 : B2_TILE_128x128;
+  if constexpr (kEpi == Epi::kPlain || kEpi == Epi::kGatedResidual) {
+    // K shared by a cluster: one round of tiles that leave half of the SMs or more idle otherwise.
+    double least = std::min(pair, std::min(big, small));
+    const auto offer = [&](int tile, double fixed, double per_block, std::int64_t tiles, int split, int resident) {
+      const double c = fixed + per_block * static_cast<double>((k_blocks + split - 1) / split);
+      if (k_blocks >= 2 * split && tiles <= resident && c < least) least = c, best = tile;
+    };
+    const std::int64_t tiles128 = m_tiles * n128, pairs = (m_tiles + 1) / 2 * n256;
+    if (tiles128 <= sms / 2) offer(kTile128x2, kSmall.fixed + 4, kSmall.per_block, tiles128, 2, resident_clusters<128, kEpi, 1, 2>());
+    if (pairs <= sms / 4) offer(kTilePairs2, kPair.fixed + 4, kPair.per_block, pairs, 2, resident_clusters<256, kEpi, 2, 2>());
+    if (pairs <= sms / 8) offer(kTilePairs4, kPair.fixed + 12, kPair.per_block, pairs, 4, resident_clusters<256, kEpi, 2, 4>());
+  }
+  return best;
 }
 
 template <Epi kEpi>
@@ -997,6 +1104,11 @@ int dispatch(const char* op, const b2_int8_operands* a, const GemmParams& p, cud
   } else {
     const int t = tile != B2_TILE_AUTO ? tile : pick_tile_int8<kEpi>(p);
     if (t == B2_TILE_2CTA_256x256) return launch_kernel<256, kEpi, 2>(op, a, p, stream);
+    if constexpr (kEpi != Epi::kAcc) {
+      if (t == kTilePairs2) return launch_kernel<256, kEpi, 2, false, 2>(op, a, p, stream);
+      if (t == kTilePairs4) return launch_kernel<256, kEpi, 2, false, 4>(op, a, p, stream);
+      if (t == kTile128x2) return launch_kernel<128, kEpi, 1, false, 2>(op, a, p, stream);
+    }
     return t == B2_TILE_128x256 ? launch_kernel<256, kEpi, 1>(op, a, p, stream) : launch_kernel<128, kEpi, 1>(op, a, p, stream);
   }
 }
