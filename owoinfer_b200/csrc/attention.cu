@@ -767,6 +767,7 @@ struct AttnArgs {
   __nv_bfloat16* out;
   std::int64_t out_row, out_head;
   int heads, q_blocks, k_blocks;
+  int batch, q_tiles;  // sequences; query tiles of the longest
   float scale_log2;  // sm_scale * log2(e)
   float p_offset;
   int hand_over;  // let the next kernel start before this one has finished (see kHandOverRows)
@@ -800,6 +801,42 @@ __device__ __forceinline__ void umma_bf16(std::uint32_t d_tmem, std::uint64_t a_
       : "memory");
 }
 
+// Which (query tile, head, sequence) a CTA works on, and where the sequence's queries and keys lie. kByLength: a flat grid
+// instead of (tiles, heads, sequences), for 2 to 32 sequences (a lane each): longest sequence first, by keys and then by
+// index, so that the short ones fill the last round; ids without a tile come last. See the launch for when.
+// Called by whole warps; false: no tile.
+template <bool kByLength>
+struct TileOfCta {
+  int bq, h, b, q_start, qo_len, k_start, kv_len;
+  __device__ __forceinline__ bool find(const AttnArgs& a, int lane) {
+    if constexpr (!kByLength) {
+      bq = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+      q_start = a.cu_q[b], qo_len = a.cu_q[b + 1] - q_start;
+      k_start = a.cu_k[b], kv_len = a.cu_k[b + 1] - k_start;
+      return bq * kTileQ < qo_len;
+    } else {
+      const int id = static_cast<int>(blockIdx.x);
+      const bool on = lane < a.batch;
+      const int q_at = on ? a.cu_q[lane] : 0, q_len = on ? a.cu_q[lane + 1] - q_at : 0;
+      const int k_at = on ? a.cu_k[lane] : 0, keys = on ? a.cu_k[lane + 1] - k_at : -1;
+      const int tiles = min(max(0, q_len + kTileQ - 1) / kTileQ, a.q_tiles);
+      int first = 0, total = 0;  // tiles (of one head) ahead of this lane's sequence, and of all
+      for (int i = 0; i < a.batch; ++i) {
+        const int k = __shfl_sync(0xffffffffu, keys, i), t = __shfl_sync(0xffffffffu, tiles, i);
+        if (k > keys || (k == keys && i < lane)) first += t;
+        total += t;
+      }
+      if (id >= total * a.heads) return false;
+      b = __ffs(__ballot_sync(0xffffffffu, on && id >= first * a.heads && id < (first + tiles) * a.heads)) - 1;
+      const auto of_b = [&](int v) { return __shfl_sync(0xffffffffu, v, b); };
+      const int at = id - of_b(first) * a.heads, n = of_b(tiles);
+      bq = at % n, h = at / n;
+      q_start = of_b(q_at), qo_len = of_b(q_len), k_start = of_b(k_at), kv_len = of_b(keys);
+      return true;
+    }
+  }
+};
+
 // One CTA per (128 query rows, head, sequence), two CTAs per SM. K and V arrive in 128-key tiles; the tensor work runs in
 // 64-key sub-tiles u = 0, 1, ... (one K scale block each) with the score accumulator double-buffered in TMEM, so the MMA
 // warp computes S(u + 1) while the softmax warps turn S(u) into P(u):
@@ -815,17 +852,16 @@ __device__ __forceinline__ void umma_bf16(std::uint32_t d_tmem, std::uint64_t a_
 //                 it took; without P it is 860. Kernel alone at 2 x 8192 tokens: 1212 -> 1166 us (1414 TOP/s), at 20480 keys
 //                 3649 -> 3516 us, at 4096 keys 194 -> 186 us; same bits.
 // kDump: the instantiation behind b2_attention_q8_debug_scores, which also stores one tile's raw integer scores.
-template <bool kDump>
+template <bool kDump, bool kByLength>
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const AttnArgs a) {
   wait_for_predecessors();
-  const int bq = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int q_start = a.cu_q[b], qo_len = a.cu_q[b + 1] - q_start;
-  const int k_start = a.cu_k[b], kv_len = a.cu_k[b + 1] - k_start;
-  const int q0 = bq * kTileQ;
-  if (q0 >= qo_len) return;  // uniform per CTA, before any barrier or allocation
   const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
+  TileOfCta<kByLength> tile;
+  if (!tile.find(a, lane)) return;  // uniform per CTA, before any barrier or allocation
+  const int bq = tile.bq, h = tile.h, b = tile.b, q_start = tile.q_start, qo_len = tile.qo_len, k_start = tile.k_start, kv_len = tile.kv_len;
+  const int q0 = bq * kTileQ;
   if (kv_len == 0) {
     // No keys: zero output rows.
     const int rows = min(kTileQ, qo_len - q0);
@@ -1450,6 +1486,7 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   a.cu_q = cu_seqlens_q, a.cu_k = cu_seqlens_k;
   a.out = static_cast<__nv_bfloat16*>(out->data), a.out_row = out->row_stride, a.out_head = out->head_stride;
   a.heads = static_cast<int>(heads), a.q_blocks = l.q_blocks, a.k_blocks = l.k_blocks;
+  a.batch = batch, a.q_tiles = (max_seqlen + kTileQ - 1) / kTileQ;
   a.scale_log2 = scale * 1.44269504088896340736f;
   a.p_offset = p_offset_of(p_range);
   a.hand_over = total_q <= kHandOverRows;
@@ -1464,12 +1501,19 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     a.trace = static_cast<long long*>(tp);
   }
 #endif
-  const auto kernel = dump != nullptr ? attention_kernel<true> : attention_kernel<false>;
+  // Longest sequence first where lengths differ much, i.e. where the keys are well below batch x the longest: in batch order
+  // sequences of 1039, 777, 2500 and 64 keys left the 480 CTAs of the longest for the end, with a thousand empty ones among
+  // them (121 us; by length 107). Of nearly equal lengths it gains nothing, and finding the tile costs each CTA some loads and
+  // shuffles (1165 + 1034 + 1165 keys: 70 us, by length 71).
+  const bool by_length = dump == nullptr && batch > 1 && batch <= 32 && 100 * total_k < 85LL * batch * max_seqlen;
+  const auto kernel = dump != nullptr ? attention_kernel<true, false> : by_length ? attention_kernel<false, true> : attention_kernel<false, false>;
   if (const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
       e != cudaSuccess) {
     return fail_cuda(op, e);
   }
-  const dim3 grid((max_seqlen + kTileQ - 1) / kTileQ, static_cast<unsigned>(heads), batch);
+  // (2^31 tiles, more than a flat grid holds, want a workspace of 500 GB.)
+  const dim3 grid = by_length ? dim3(static_cast<unsigned>(static_cast<std::int64_t>(a.q_tiles) * heads * batch))
+                              : dim3(a.q_tiles, static_cast<unsigned>(heads), batch);
   return enqueue(op, kernel, grid, kAttnThreads, kAttnSmem, st, 1, map_q, map_k, map_v, a);
 }
 }  // namespace

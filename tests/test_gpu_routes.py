@@ -1,4 +1,5 @@
 """Routes that a rule on sizes picks, against the general route of the same call: the same bits."""
+import numpy as np
 import pytest
 import torch
 
@@ -34,4 +35,22 @@ def test_gemm_tiles_that_share_k_give_the_bits_of_whole_tiles(ops, m, n, k):
     ops.int8_gemm_gated_residual(x, xs, w, ws, gate, res)
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     assert torch.equal(res.view(torch.int16), want_res.view(torch.int16))
+    assert ops.kernel_status() == (0, 0)
+
+
+@pytest.mark.parametrize("lens,keys", [([300, 64, 700, 129], None), ([1, 0, 257, 40], [513, 70, 64, 900]), ([130] + [40] * 31, None), ([200] + [33] * 33, None)])
+def test_attention_of_a_batch_is_that_of_its_sequences(ops, lens, keys):
+    """Sequences of different lengths are handed out longest first up to 32 of them, in batch order beyond."""
+    heads, keys = 2, keys or lens
+    q = torch.randn((sum(lens), heads, 128), device="cuda", generator=_gen(5)).bfloat16()
+    k, v = (torch.randn((sum(keys), heads, 128), device="cuda", generator=_gen(s)).bfloat16() for s in (6, 7))
+    cu = lambda n: torch.tensor(np.concatenate([[0], np.cumsum(n)]), dtype=torch.int32, device="cuda")
+    out, want = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
+    ops.attention_q8(q, k, v, out, cu(lens), cu(keys), max(lens + keys), ops.SM_SCALE)
+    a = b = 0
+    for n, m in zip(lens, keys):
+        if n > 0:
+            ops.attention_q8(q[a:a + n], k[b:b + m], v[b:b + m], want[a:a + n], cu([n]), cu([m]), max(n, m), ops.SM_SCALE)
+        a, b = a + n, b + m
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
     assert ops.kernel_status() == (0, 0)
