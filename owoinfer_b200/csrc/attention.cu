@@ -1,6 +1,6 @@
 // SageAttention-style 8-bit attention for sm_100a, plus the MOSS QK-norm + RoPE and RoPE-table kernels that feed it.
 //
-//   pre-pass (HBM-bound, 128-bit accesses)
+//   pre-pass (HBM-bound, 128-bit accesses; all of it in one launch for sequences of up to 512 tokens)
 //     prologue   (fused QK-norm + RoPE only) per (32 tokens, head): RMS-norm + RoPE of q and k, k written back,
 //                Q quantised
 //     stats      per (512-key chunk, head, sequence): partial per-channel K sums and V |max| in a fixed order
@@ -651,6 +651,197 @@ __global__ void __launch_bounds__(256) quant_kv_kernel(const PrepArgs p) {
         make_uint2(pack_i8x4(x[i][0] * ks, x[i][1] * ks, x[i][2] * ks, x[i][3] * ks),
                    pack_i8x4(x[i][4] * ks, x[i][5] * ks, x[i][6] * ks, x[i][7] * ks));
     const std::uint32_t w[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[2 * j] = __uint_as_float(w[j] << 16) * recp[2 * j];
+      v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u) * recp[2 * j + 1];
+    }
+    *reinterpret_cast<uint2*>(p.v8 + o) = make_uint2(e4m3x4(v[0], v[1], v[2], v[3]), e4m3x4(v[4], v[5], v[6], v[7]));
+  }
+}
+
+// The whole pre-pass of runs whose sequences fit one statistics chunk: a cluster per (head, sequence), a CTA per 64 tokens,
+// so that prologue, statistics, finalize and both quantisers are one launch and q, k and v are read once. The arithmetic and
+// its order are those of the four kernels: K sums in 16 row chains over the sequence, each channel's by the CTA that owns
+// its 16-channel group (from every CTA's rows in distributed shared memory), the chains added in order. Bound by latency: at 297 rows the four
+// launches took 17.5 us of a 127 us block, which this one brings to 122; at 320 + 266 rows 164 to 159.
+__device__ __forceinline__ std::uint32_t ld_cluster_u16(std::uint32_t addr) {
+  std::uint16_t v;
+  asm volatile("ld.shared::cluster.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster_f32(std::uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_cluster_f32(std::uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__global__ void __launch_bounds__(512, 2) short_prepass_kernel(const PrepArgs p) {
+  dependents_may_start();
+  __shared__ __align__(16) uint4 s_k[64 * 16];  // the CTA's k rows after QK-norm + RoPE, bf16 [64, 128]
+  __shared__ __align__(16) float s_red[16][kHeadDim];
+  __shared__ __align__(16) float s_vmax[kHeadDim], s_mean[kHeadDim], s_recp[kHeadDim];
+  __shared__ float s_w[3][16];
+  const int bx = blockIdx.x, h = blockIdx.y, b = blockIdx.z, ctas = gridDim.x;
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 15, row = tid >> 4, warp = tid >> 5;
+  const auto quad = [](uint4 v, std::uint32_t (&o)[4]) { o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w; };
+  wait_for_predecessors();
+  const int start = p.cu[b], len = min(p.cu[b + 1] - start, 64 * ctas);
+  const int pair = (lane & 7) * 8;
+  if (bx == 0 && b == p.batch - 1) {
+    // As in quant_kv_kernel: rows of V behind the last sequence that its last 128-key tile brings along.
+    const std::int64_t end = static_cast<std::int64_t>(start) + len, stop = min(end + 127, p.key_rows);
+    for (std::int64_t r = end + row; r < stop; r += 32) *reinterpret_cast<uint2*>(p.v8 + (r * p.heads + h) * kHeadDim + lane * 8) = make_uint2(0u, 0u);
+  }
+  uint4 vr[2];
+  float vmax[8] = {};
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {  // 32 tokens = one Q block each
+    const int t = bx * 64 + hh * 32 + row;
+    const bool valid = t < len;
+    const std::int64_t tok = static_cast<std::int64_t>(start) + t;
+    uint4 xr = make_uint4(0, 0, 0, 0), kr = xr, sr = xr, cr = xr;
+    vr[hh] = xr;
+    __nv_bfloat16* k_at = p.k + tok * p.k_row + h * p.k_head + lane * 8;
+    if (valid) {
+      xr = *reinterpret_cast<const uint4*>(p.q + tok * p.q_row + h * p.q_head + lane * 8);
+      kr = *reinterpret_cast<const uint4*>(k_at);
+      vr[hh] = *reinterpret_cast<const uint4*>(p.v + tok * p.v_row + h * p.v_head + lane * 8);
+      sr = *reinterpret_cast<const uint4*>(p.table + tok * p.table_row + pair);
+      cr = *reinterpret_cast<const uint4*>(p.table + tok * p.table_row + 64 + pair);
+    }
+    std::uint32_t x[4], kx[4], si[4], co[4], w[4], qy[4], ky[4];
+    quad(xr, x), quad(kr, kx), quad(sr, si), quad(cr, co);
+    if (lane < 8) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) si[i] ^= 0x80008000u;
+    }
+    quad(*reinterpret_cast<const uint4*>(p.q_norm + lane * 8), w);
+    norm_rope_row(x, w, si, co, p.norm_factor, qy);
+    quad(*reinterpret_cast<const uint4*>(p.k_norm + lane * 8), w);
+    norm_rope_row(kx, w, si, co, p.norm_factor, ky);
+    if (valid) *reinterpret_cast<uint4*>(k_at) = make_uint4(ky[0], ky[1], ky[2], ky[3]);
+    s_k[(hh * 32 + row) * 16 + lane] = make_uint4(ky[0], ky[1], ky[2], ky[3]);
+    float q[8], qmax = 0.0000001f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      q[2 * i] = __uint_as_float(qy[i] << 16);
+      q[2 * i + 1] = __uint_as_float(qy[i] & 0xFFFF0000u);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) qmax = fmaxf(qmax, fabsf(q[j]));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) qmax = fmaxf(qmax, __shfl_xor_sync(0xffffffffu, qmax, off));
+    if ((tid & 31) == 0) s_w[hh][warp] = qmax;
+    __syncthreads();
+    qmax = s_w[hh][0];
+#pragma unroll
+    for (int i = 1; i < 16; ++i) qmax = fmaxf(qmax, s_w[hh][i]);
+    if (tid == 0) p.q_scale[(static_cast<std::int64_t>(b) * p.heads + h) * p.q_blocks + bx * 2 + hh] = qmax / 127.0f;
+    const float qs = 127.0f / qmax;
+    if (valid) {
+      *reinterpret_cast<uint2*>(p.q_i8 + (tok * p.heads + h) * kHeadDim + lane * 8) =
+          make_uint2(pack_i8x4(q[0] * qs, q[1] * qs, q[2] * qs, q[3] * qs), pack_i8x4(q[4] * qs, q[5] * qs, q[6] * qs, q[7] * qs));
+    }
+    const std::uint32_t vw[4] = {vr[hh].x, vr[hh].y, vr[hh].z, vr[hh].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      vmax[2 * i] = fmaxf(vmax[2 * i], fabsf(__uint_as_float(vw[i] << 16)));
+      vmax[2 * i + 1] = fmaxf(vmax[2 * i + 1], fabsf(__uint_as_float(vw[i] & 0xFFFF0000u)));
+    }
+  }
+  // Q blocks past the last CTA's hold no tokens.
+  for (int i = 2 * ctas + tid; bx == 0 && i < p.q_blocks; i += 512) {
+    p.q_scale[(static_cast<std::int64_t>(b) * p.heads + h) * p.q_blocks + i] = 0.0000001f / 127.0f;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    vmax[j] = fmaxf(vmax[j], __shfl_xor_sync(0xffffffffu, vmax[j], 16));
+    if ((tid & 16) == 0) s_red[warp][lane * 8 + j] = vmax[j];
+  }
+  __syncthreads();
+  if (tid < kHeadDim) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, s_red[i][tid]);
+    s_vmax[tid] = m;
+  }
+  cluster_sync_all();
+  // The channel groups of this CTA, two at a time (256 threads = 16 row chains x 16 channels).
+  const int half = tid >> 8, chain = (tid & 255) >> 4;
+  for (int g = bx + ctas * half; g < 8; g += 2 * ctas) {
+    const int ch = g * 16 + lane;
+    float sum = 0.f;
+    for (int t0 = chain; t0 < len; t0 += 16 * 4) {  // a CTA's 64 rows: four of the chain, whose loads go ahead of the sums
+      const std::uint32_t rows = map_to_cta(smem_u32(s_k), static_cast<std::uint32_t>(t0 >> 6)) + ch * 2;
+      std::uint32_t k[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) k[u] = ld_cluster_u16(rows + (chain + 16 * u) * (kHeadDim * 2));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (t0 + 16 * u < len) sum += __uint_as_float(k[u] << 16);
+      }
+    }
+    s_red[chain][half * 64 + lane] = sum;
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + half) : "memory");
+    if (chain == 0) {
+      float s = 0.f, a = 0.f;
+      for (int r = 0; r < 16; ++r) s += s_red[r][half * 64 + lane];
+      for (int c = 0; c < ctas; ++c) a = fmaxf(a, ld_cluster_f32(map_to_cta(smem_u32(&s_vmax[ch]), static_cast<std::uint32_t>(c))));
+      const float mean = len > 0 ? rbf(s / static_cast<float>(len)) : 0.f, recp = a > 0.f ? p.v_range / a : 1.f;
+      const std::int64_t at = (static_cast<std::int64_t>(b) * p.heads + h) * kHeadDim + ch;
+      p.k_mean[at] = mean;
+      p.v_scale[at] = a > 0.f ? a / p.v_range : 1.f;
+      p.v_recp[at] = recp;
+      for (int c = 0; c < ctas; ++c) {
+        st_cluster_f32(map_to_cta(smem_u32(&s_mean[ch]), static_cast<std::uint32_t>(c)), mean);
+        st_cluster_f32(map_to_cta(smem_u32(&s_recp[ch]), static_cast<std::uint32_t>(c)), recp);
+      }
+    }
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + half) : "memory");
+  }
+  cluster_sync_all();
+  float mean[8];
+  *reinterpret_cast<float4*>(mean) = *reinterpret_cast<const float4*>(s_mean + lane * 8);
+  *reinterpret_cast<float4*>(mean + 4) = *reinterpret_cast<const float4*>(s_mean + lane * 8 + 4);
+  float x[2][8], amax = 0.0000001f;
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const uint4 kr = s_k[(hh * 32 + row) * 16 + lane];
+    const std::uint32_t w[4] = {kr.x, kr.y, kr.z, kr.w};
+    const bool valid = bx * 64 + hh * 32 + row < len;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // An absent key contributes 0 (not 0 - mean) to the block maximum.
+      x[hh][2 * j] = valid ? __uint_as_float(w[j] << 16) - mean[2 * j] : 0.f;
+      x[hh][2 * j + 1] = valid ? __uint_as_float(w[j] & 0xFFFF0000u) - mean[2 * j + 1] : 0.f;
+      amax = fmaxf(amax, fmaxf(fabsf(x[hh][2 * j]), fabsf(x[hh][2 * j + 1])));
+    }
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+  if ((tid & 31) == 0) s_w[2][warp] = amax;
+  __syncthreads();
+  amax = s_w[2][0];
+#pragma unroll
+  for (int i = 1; i < 16; ++i) amax = fmaxf(amax, s_w[2][i]);
+  if (tid == 0) p.k_scale[(static_cast<std::int64_t>(b) * p.heads + h) * p.k_blocks + bx] = amax / 127.0f;
+  const float ks = 127.0f / amax;
+  float recp[8];
+  *reinterpret_cast<float4*>(recp) = *reinterpret_cast<const float4*>(s_recp + lane * 8);
+  *reinterpret_cast<float4*>(recp + 4) = *reinterpret_cast<const float4*>(s_recp + lane * 8 + 4);
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const int t = bx * 64 + hh * 32 + row;
+    if (t >= len) continue;
+    const std::int64_t o = ((static_cast<std::int64_t>(start) + t) * p.heads + h) * kHeadDim + lane * 8;
+    *reinterpret_cast<uint2*>(p.k_i8 + o) =
+        make_uint2(pack_i8x4(x[hh][0] * ks, x[hh][1] * ks, x[hh][2] * ks, x[hh][3] * ks),
+                   pack_i8x4(x[hh][4] * ks, x[hh][5] * ks, x[hh][6] * ks, x[hh][7] * ks));
+    const std::uint32_t w[4] = {vr[hh].x, vr[hh].y, vr[hh].z, vr[hh].w};
     float v[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1449,7 +1640,6 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     if (rows->slot_run || p.tap != nullptr) p.all_rows = total_q;
   }
   const bool slots = p.slot[0] != nullptr || p.slot[1] != nullptr;
-  const dim3 stats_grid(l.chunks, static_cast<unsigned>(heads), batch);
   if (norm_rope != nullptr) {
     const std::int64_t norm_rows = total_q * heads;
     p.q_norm = static_cast<const __nv_bfloat16*>(norm_rope->q_norm);
@@ -1457,21 +1647,29 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     p.table = static_cast<const __nv_bfloat16*>(norm_rope->table);
     p.table_row = norm_rope->table_ld;
     p.norm_factor = static_cast<float>(norm_rows) / static_cast<float>(norm_rows * kHeadDim);
-    PrepArgs own = p;  // queries and the key rows of the same tokens
-    own.cu = cu_seqlens_q, own.k = p.k + p.own0 * p.k_row;
-    const auto kernel = p.all_rows > 0 ? norm_rope_quant_q_kernel<true> : norm_rope_quant_q_kernel<false>;
-    if (const int rc = enqueue(op, kernel, dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st, 1, own)) return rc;
   }
-  if (const int rc = enqueue(op, slots ? stats_kernel<true> : stats_kernel<false>, stats_grid, 256, 0, st, 1, p)) return rc;
-  if (const int rc = enqueue(op, finalize_kernel, dim3(static_cast<unsigned>(heads), batch), kHeadDim, 0, st, 1, p)) return rc;
-  if (norm_rope == nullptr) {
-    PrepArgs pq = p;
-    pq.cu = cu_seqlens_q;
-    if (const int rc = enqueue(op, quant_q_kernel, dim3(l.q_blocks, static_cast<unsigned>(heads), batch), 512, 0, st, 1, pq)) return rc;
+  const unsigned h = static_cast<unsigned>(heads);
+  if (norm_rope != nullptr && max_seqlen <= kStatsChunk && !slots && p.all_rows == 0 && cu_seqlens_q == cu_seqlens_k) {
+    // Sequences of one statistics chunk whose rows are all their own.
+    if (const int rc = enqueue(op, short_prepass_kernel, dim3(l.k_blocks, h, batch), 512, 0, st, l.k_blocks, p)) return rc;
+  } else {
+    if (norm_rope != nullptr) {
+      PrepArgs own = p;  // queries and the key rows of the same tokens
+      own.cu = cu_seqlens_q, own.k = p.k + p.own0 * p.k_row;
+      const auto kernel = p.all_rows > 0 ? norm_rope_quant_q_kernel<true> : norm_rope_quant_q_kernel<false>;
+      if (const int rc = enqueue(op, kernel, dim3(l.q_blocks, h, batch), 512, 0, st, 1, own)) return rc;
+    }
+    if (const int rc = enqueue(op, slots ? stats_kernel<true> : stats_kernel<false>, dim3(l.chunks, h, batch), 256, 0, st, 1, p)) return rc;
+    if (const int rc = enqueue(op, finalize_kernel, dim3(h, batch), kHeadDim, 0, st, 1, p)) return rc;
+    if (norm_rope == nullptr) {
+      PrepArgs pq = p;
+      pq.cu = cu_seqlens_q;
+      if (const int rc = enqueue(op, quant_q_kernel, dim3(l.q_blocks, h, batch), 512, 0, st, 1, pq)) return rc;
+    }
+    // (A tapped run reads no slots.)
+    const auto quant_kv = p.tap != nullptr ? quant_kv_kernel<false, true> : slots ? quant_kv_kernel<true, false> : quant_kv_kernel<false, false>;
+    if (const int rc = enqueue(op, quant_kv, dim3(l.k_blocks, h, batch), 256, 0, st, 1, p)) return rc;
   }
-  // (A tapped run reads no slots.)
-  const auto quant_kv = p.tap != nullptr ? quant_kv_kernel<false, true> : slots ? quant_kv_kernel<true, false> : quant_kv_kernel<false, false>;
-  if (const int rc = enqueue(op, quant_kv, dim3(l.k_blocks, static_cast<unsigned>(heads), batch), 256, 0, st, 1, p)) return rc;
   if (prepass_only) return B2_OK;
 
   CUtensorMap map_q, map_k, map_v;

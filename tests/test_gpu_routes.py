@@ -38,6 +38,31 @@ def test_gemm_tiles_that_share_k_give_the_bits_of_whole_tiles(ops, m, n, k):
     assert ops.kernel_status() == (0, 0)
 
 
+@pytest.mark.parametrize("lens", [[1], [33], [64], [65], [297], [512], [320, 266], [17, 0, 512], [100, 448, 3, 64, 449]])
+def test_prepass_of_short_sequences_in_one_launch(ops, lens):
+    """max_seqlen up to 512: the pre-pass is one launch. The same call with a larger max_seqlen takes the separate kernels."""
+    heads, total, batch = 3, sum(lens), len(lens)
+    qkv = torch.randn((total, 3 * heads * 128), device="cuda", generator=_gen(total)).bfloat16()
+    norms = [(1 + 0.1 * torch.randn(128, device="cuda", generator=_gen(i))).bfloat16() for i in (1, 2)]
+    table = torch.cat([ops.moss_rope_table(1, 1, n - 1) for n in lens if n > 0]).contiguous()
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    got = []
+    for longest in (max(lens), 1025):
+        x = qkv.clone()
+        q, k, v = (x[:, i * heads * 128:(i + 1) * heads * 128].unflatten(1, (heads, 128)) for i in range(3))
+        l = ops.attention_q8_layout(total, total, batch, longest, heads)
+        ws = torch.full((l.total,), 0x55, dtype=torch.uint8, device="cuda")
+        ops.attention_q8_preprocess(q, k, v, cu, cu, longest, workspace=ws, norm_rope=(norms[0], norms[1], table))
+        cut = lambda at, *shape: ws[at:at + int(np.prod(shape))].view(*shape).clone()
+        rows = [cut(at, total * heads, 128) for at in (l.q_i8, l.k_i8, l.v8)]
+        stats = [cut(at, batch * heads, 512) for at in (l.k_mean, l.v_scale, l.v_recp)]
+        qs, ks = cut(l.q_scale, batch * heads, 4 * l.q_blocks), cut(l.k_scale, batch * heads, 4 * l.k_blocks)
+        n = (max(lens) + 127) // 128 * 16, (max(lens) + 63) // 64 * 4
+        got.append([x.view(torch.int16), *rows, *stats, qs[:, :n[0]], ks[:, :n[1]]])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("lens,keys", [([300, 64, 700, 129], None), ([1, 0, 257, 40], [513, 70, 64, 900]), ([130] + [40] * 31, None), ([200] + [33] * 33, None)])
 def test_attention_of_a_batch_is_that_of_its_sequences(ops, lens, keys):
     """Sequences of different lengths are handed out longest first up to 32 of them, in batch order beyond."""
