@@ -22,7 +22,10 @@ ATTENTION_Q8_FP8_F32ACC = 3
 
 
 def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    if not torch.cuda.is_initialized():
+        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # The same handle without the Stream object around it, whose making is a good part of a small call.
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _ptr(t) -> C.c_void_p:
@@ -459,12 +462,11 @@ def guided_velocity_step(v_cond, x=None, v_uncond=None, v_skip=None, v_prev=None
                          h=0.0, a=0.0, b=0.0, update=0):
     """One pass: guidance (cfg when v_uncond is given, slg when v_skip is given), optional store of the guided velocity,
     and the Euler (update 1) or Adams-Bashforth (update 2) step of x."""
-    g = _lib.GuidedStep()
-    g.struct_size = C.sizeof(_lib.GuidedStep)
-    p = lambda t: None if t is None else t.data_ptr()
-    g.x, g.v_cond, g.v_uncond, g.v_skip, g.v_prev, g.v_out = p(x), p(v_cond), p(v_uncond), p(v_skip), p(v_prev), p(v_out)
-    g.cfg_scale, g.slg_scale, g.h, g.a, g.b = cfg_scale, slg_scale, h, a, b
-    g.cfg, g.slg, g.update, g.n = int(v_uncond is not None), int(v_skip is not None), update, v_cond.numel()
+    # (Filled in one go: the kernel is a microsecond or two, so the host's side of this call is most of its time.)
+    g = _lib.GuidedStep(C.sizeof(_lib.GuidedStep), None if x is None else x.data_ptr(), None if v_cond is None else v_cond.data_ptr(),
+                        None if v_uncond is None else v_uncond.data_ptr(), None if v_skip is None else v_skip.data_ptr(),
+                        None if v_prev is None else v_prev.data_ptr(), None if v_out is None else v_out.data_ptr(), cfg_scale, slg_scale,
+                        h, a, b, int(v_uncond is not None), int(v_skip is not None), update, v_cond.numel())
     check(_lib.lib().b2_guided_velocity_step(C.byref(g), _stream()))
     return x if update else v_out
 
