@@ -19,7 +19,7 @@ SOFTMAX = [(4, "loop top"), (8, "scale of the sub-tile ready"), (0, "S(u) in reg
            (9, "vote: nothing to rescale"), (2, "pass stands"), (10, "P(u) in tensor memory"), (11, "tcgen05 fence + __syncwarp"),
            (3, "arrived on p_full(u)"), (12, "S(u+1) computed, P.V(u-1) landed (s_step wait)"), (13, "loads of S(u+1) issued"),
            (14, "headroom check done")]
-MMA = [(5, "p_full(u) seen"), (6, "P.V(u) issued"), (7, "Q.K^T(u+2) issued, step committed")]
+MMA = [(5, "p_full(u) seen"), (7, "P.V(u) and Q.K^T(u+2) issued, step committed")]
 
 
 def build_trace() -> str:
@@ -57,7 +57,6 @@ def main() -> None:
     if fn(buf, 4096) != 0:
         raise RuntimeError("the trace could not be read")
     full = np.array(buf[:4096], dtype=np.int64).reshape(-1, 16)
-    print("start-up issues with idle softmax warps: Q.K^T(0) incl. the wait for K", int(full[200, 1] - full[200, 0]), "clocks, Q.K^T(1)", int(full[200, 2] - full[200, 1]), "clocks")
     a = full[:128]
     u = np.arange(9, 120)
     med = lambda x: float(np.median(x))

@@ -1137,77 +1137,72 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     const std::uint64_t dv0 = umma_desc_sw128(v_smem(0)), dv1 = umma_desc_sw128(v_smem(1));
     // 64 keys = 64 rows of 128 bytes of a K or V tile: 8192 bytes, 512 in the descriptors' 16-byte units.
     constexpr std::uint32_t kHalfTile = 64 * 128 / 16;
-    // S(u % 2) = [12582912.0f +] Q · K(u)^T. The K tile goes back to the TMA warp after its second half.
-    const auto issue_qk = [&](int u) -> bool {
-      const int s = (u >> 1) % kKvStages;
-      bool got = true;
-      if ((u & 1) == 0) got = wait_bar(smem_u32(&s_k_full[s]), ((u >> 1) / kKvStages) & 1u, abort_word);
-      if (__any_sync(0xffffffffu, !got)) return false;
-      tc_fence_after();
-      if (elect_one()) {
-        const std::uint32_t d_s = tmem_s + static_cast<std::uint32_t>(u & 1) * kSubK;
-        // The constant operand serves as A (128 rows) and as B (its first 64 rows): every row holds the same 16 values.
-        if (B2_ATTN_CONST_BIAS) umma_bf16(d_s, dconst, dconst, idesc_bias, 0u);
-        const std::uint64_t d = (s != 0 ? dk1 : dk0) + (u & 1) * kHalfTile;
+    // S(u % 2) = [12582912.0f +] Q · K(u)^T, by the elected lane. The constant operand serves as A (128 rows) and as B (its
+    // first 64 rows): every row holds the same 16 values.
+    const auto issue_scores = [&](std::uint32_t d_s, std::uint64_t dk) {
+      if (B2_ATTN_CONST_BIAS) umma_bf16(d_s, dconst, dconst, idesc_bias, 0u);
 #pragma unroll
-        for (int k4 = 0; k4 < 4; ++k4) {
-          umma_i8(d_s, dq + 2u * k4, d + 2u * k4, idesc_qk, (B2_ATTN_CONST_BIAS || k4 != 0) ? 1u : 0u);
-        }
-        if ((u & 1) != 0 || u + 1 >= n_sub) tc_commit(smem_u32(&s_k_empty[s]));
-        if (u < 2) tc_commit(smem_u32(&s_step[u]));  // start-up: S(0) and S(1) are the first completions of the two barriers
-      }
-      __syncwarp();
-      return true;
+      for (int k4 = 0; k4 < 4; ++k4) umma_i8(d_s, dq + 2u * k4, dk + 2u * k4, idesc_qk, (B2_ATTN_CONST_BIAS || k4 != 0) ? 1u : 0u);
     };
-    bool ok = wait_bar(smem_u32(&s_q_full), 0, abort_word) && wait_bar(smem_u32(&s_s_ready), 0, abort_word);
-    ok = !__any_sync(0xffffffffu, !ok);
+    bool got = wait_bar(smem_u32(&s_q_full), 0, abort_word) && wait_bar(smem_u32(&s_s_ready), 0, abort_word) &&
+               wait_bar(smem_u32(&s_k_full[0]), 0, abort_word);
+    bool ok = !__any_sync(0xffffffffu, !got);
     tc_fence_after();
-#ifdef B2_ATTN_TRACE
-    // Tracing only: wait for both K halves' tile first, then time the two start-up issues (the softmax warps are idle).
-    if (tracing) a.trace[200 * 16 + 0] = clock64();
-#endif
-    ok = ok && issue_qk(0);
-#ifdef B2_ATTN_TRACE
-    if (tracing) a.trace[200 * 16 + 1] = clock64();
-#endif
-    if (ok && n_sub > 1) ok = issue_qk(1);
-#ifdef B2_ATTN_TRACE
-    if (tracing) a.trace[200 * 16 + 2] = clock64();
-#endif
-    for (int u = 0; ok && u < n_sub; ++u) {
-      const int s = (u >> 1) % kKvStages;
-      bool got = true;
-      if ((u & 1) == 0) got = wait_bar(smem_u32(&s_v_full[s]), ((u >> 1) / kKvStages) & 1u, abort_word);
-      // The softmax warps have consumed S(u) and written P(u).
-      got = got && wait_bar_relaxed<B2_MMA_SLEEP_NS>(smem_u32(&s_p_full[u & 1]), (u >> 1) & 1u, abort_word);
-      if (__any_sync(0xffffffffu, !got)) break;
-      tc_fence_after();
-      TRACE(5);
-      if (elect_one()) {
+    if (ok && elect_one()) {  // start-up: S(0) and S(1) are the first completions of the two barriers
+      issue_scores(tmem_s, dk0);
+      tc_commit(smem_u32(&s_step[0]));
+      if (n_sub > 1) {
+        issue_scores(tmem_s + kSubK, dk0 + kHalfTile);
+        tc_commit(smem_u32(&s_step[1]));
+      }
+      tc_commit(smem_u32(&s_k_empty[0]));
+    }
+    __syncwarp();
+    // Step u, once the softmax warps have consumed S(u) and written P(u): O += P(u) · V(u), then S(u + 2), whose columns hold
+    // P(u); one completion for both. All of a step is issued in one go behind its waits: with the vote, the fence and the
+    // election once for P·V and once for the scores the warp needed 1580 clocks a step even with softmax warps that did next
+    // to nothing, now 1240 (8192 + 8192 keys: 1033 -> 893 us in that timing-only build, 1174 -> 1159 us in the product,
+    // 512 -> 497 us on peaked scores at 4378 + 4106). (By a single lane instead of the whole warp: 1216 us.)
+    for (int t = 0; ok && t < n_tiles; ++t) {
+      const int s = t % kKvStages, s_next = (t + 1) % kKvStages;
 #pragma unroll
-        for (int k2 = 0; k2 < 2; ++k2) {
+      for (int h = 0; h < 2; ++h) {
+        const int u = 2 * t + h;
+        if (u >= n_sub) break;
+        const bool more = u + 2 < n_sub;
+        got = true;
+        if (h == 0) {
+          got = wait_bar(smem_u32(&s_v_full[s]), (t / kKvStages) & 1u, abort_word);
+          if (more) got = got && wait_bar(smem_u32(&s_k_full[s_next]), ((t + 1) / kKvStages) & 1u, abort_word);
+        }
+        got = got && wait_bar_relaxed<B2_MMA_SLEEP_NS>(smem_u32(&s_p_full[h]), t & 1u, abort_word);
+        ok = !__any_sync(0xffffffffu, !got);
+        if (!ok) break;
+        tc_fence_after();
+        TRACE(5);
+        if (elect_one()) {
           // P(u): the first 16 columns of S(u), 32 keys to 8 columns; V (MN-major): 32 key rows of 128 bytes (+256 per
           // step), second half of the tile at +kHalfTile.
-          umma_f8_ts(tmem_o, tmem_s + static_cast<std::uint32_t>(u & 1) * kSubK + 8u * k2,
-                     (s != 0 ? dv1 : dv0) + (u & 1) * kHalfTile + 256u * k2, idesc_pv, (u | k2) != 0 ? 1u : 0u);
+          const std::uint32_t d_s = tmem_s + static_cast<std::uint32_t>(h) * kSubK;
+          const std::uint64_t dv = (s != 0 ? dv1 : dv0) + h * kHalfTile;
+          umma_f8_ts(tmem_o, d_s, dv, idesc_pv, u != 0 ? 1u : 0u);
+          umma_f8_ts(tmem_o, d_s + 8u, dv + 256u, idesc_pv, 1u);
+          if (more) issue_scores(d_s, (s_next != 0 ? dk1 : dk0) + h * kHalfTile);
+          tc_commit(smem_u32(&s_step[h]));
+          if (h == 1 || u + 1 >= n_sub) tc_commit(smem_u32(&s_v_empty[s]));
+          if (more && (h == 1 || u + 3 >= n_sub)) tc_commit(smem_u32(&s_k_empty[s_next]));
         }
-        if ((u & 1) != 0 || u + 1 >= n_sub) tc_commit(smem_u32(&s_v_empty[s]));
-      }
-      __syncwarp();
-      TRACE(6);
-      if (u + 2 < n_sub && !issue_qk(u + 2)) break;
-      // One completion per step: P·V(u) has landed (its P buffer and O are free again) and S(u + 2) is computed.
-      if (elect_one()) tc_commit(smem_u32(&s_step[u & 1]));
-      __syncwarp();
-      TRACE(7);
+        __syncwarp();
+        TRACE(7);
 #ifdef B2_ATTN_TRACE
-      // Tracing only: when the step's MMAs have completed (the warp has nothing else to do until P(u + 1) arrives).
-      if (tracing) {
-        for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(smem_u32(&s_step[u & 1]), ((u >> 1) + 1) & 1u); ++spin) {
+        // Tracing only: when the step's MMAs have completed (the warp has nothing else to do until P(u + 1) arrives).
+        if (tracing) {
+          for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(smem_u32(&s_step[h]), (t + 1) & 1u); ++spin) {
+          }
+          TRACE(15);
         }
-        TRACE(15);
-      }
 #endif
+      }
     }
   } else {
     // Softmax: 4 warps, one thread per query row; warp w may touch TMEM lanes [32 (w % 4), +32). One pass per sub-tile:
