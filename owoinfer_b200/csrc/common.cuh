@@ -223,6 +223,18 @@ __device__ __forceinline__ bool mbar_try_wait(std::uint32_t bar, std::uint32_t p
       : "memory");
   return ok != 0;
 }
+// The same test without ever suspending the thread.
+__device__ __forceinline__ bool mbar_test_wait(std::uint32_t bar, std::uint32_t parity) {
+  std::uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // The same test, letting the hardware keep the thread suspended for up to `hint_ns` while the phase is incomplete (it
 // resumes when the phase completes): a waiting warp then issues next to no instructions.
 #ifndef B2_WAIT_HINT_NS
