@@ -110,7 +110,7 @@ typedef struct b2_int8_operands {
 } b2_int8_operands;
 
 /* quant::Int8Tile (src/kernels/quant/quant.h:77). The tcgen05 kernel has its own tiles; every tile gives the same
- * bits (the int32 sum is exact). 0 = auto. */
+ * bits (the int32 sum is exact). 0 = auto; a value that the enum does not have runs 128 x 128 (SiTU-GLU: 128 x 256). */
 typedef enum b2_int8_tile { B2_TILE_AUTO = 0, B2_TILE_128x256 = 1, B2_TILE_128x128 = 2, B2_TILE_2CTA_256x256 = 3 } b2_int8_tile;
 
 /* quant::int8_gemm (src/kernels/quant/quant.h:92): out = bf16((acc * x_scale[r]) * w_scale[c] + bias[c]).

@@ -1034,14 +1034,18 @@ int pick_tile(int tile, std::int64_t m, std::int64_t n_tiles_256) {
 struct TileCost {
   double fixed, per_block;
 };
-// Tiles whose K range a cluster shares (never asked for by a caller). Measured, 3072 columns, us (rows x K):
+// What a launch runs: the tile shape (b2_int8_tile, never AUTO) and how many CTAs (pairs) of a cluster share a tile's K range.
+// Only the choice below splits: a caller's tile argument names a shape.
+// Splits measured, 3072 columns, us (rows x K):
 //                128 x 128   pairs   128 x 128 in two   pairs in two   pairs in four
 //   100 x 12288    30.3      35.9         20.2              23.7           19.6
 //   297 x 3072     12.1      15.5         11.0              13.2
 //   297 x 8192     22.1      27.2         16.4              19.2
 //   400 x 8192     22.3      27.1                           19.5
 //   400 x 12288    30.7      36.3                           24.2
-constexpr int kTilePairs2 = 16, kTilePairs4 = 17, kTile128x2 = 18;
+struct TileChoice {
+  int tile, split;
+};
 // How many clusters of a split tile's kernel the device holds at once (asked once per device): a grid of more would run in
 // two rounds. (Clusters of four reach 132 of a B200's 148 SMs, of eight 120.)
 template <int kBN, Epi kEpi, int kCtas, int kSplit>
@@ -1069,7 +1073,7 @@ int resident_clusters() {
 }
 
 template <Epi kEpi>
-int pick_tile_int8(const GemmParams& p) {
+TileChoice pick_tile_int8(const GemmParams& p) {
   constexpr bool kSitu = kEpi == Epi::kSituGlu;
   constexpr TileCost kPair = kSitu ? TileCost{50, 1.1} : TileCost{33, 1.0}, kBig = kSitu ? TileCost{43, 1.64} : TileCost{27, 1.5}, kSmall{21, 0.95};
   const int k_blocks = (p.k + kBK - 1) / kBK, sms = sm_count();
@@ -1080,36 +1084,35 @@ int pick_tile_int8(const GemmParams& p) {
   };
   const double pair = cost(kPair, (m_tiles + 1) / 2 * n256, sms / 2), big = cost(kBig, m_tiles * n256, sms);
   const double small = kSitu ? big : cost(kSmall, m_tiles * n128, sms);
-  int best = pair <= big && pair <= small ? B2_TILE_2CTA_256x256 : big <= small ? B2_TILE_128x256 : B2_TILE_128x128;
+  TileChoice best{pair <= big && pair <= small ? B2_TILE_2CTA_256x256 : big <= small ? B2_TILE_128x256 : B2_TILE_128x128, 1};
   if constexpr (kEpi == Epi::kPlain || kEpi == Epi::kGatedResidual) {
     // K shared by a cluster: one round of tiles that leave half of the SMs or more idle otherwise.
     double least = std::min(pair, std::min(big, small));
     const auto offer = [&](int tile, double fixed, double per_block, std::int64_t tiles, int split, int resident) {
       const double c = fixed + per_block * static_cast<double>((k_blocks + split - 1) / split);
-      if (k_blocks >= 2 * split && tiles <= resident && c < least) least = c, best = tile;
+      if (k_blocks >= 2 * split && tiles <= resident && c < least) least = c, best = {tile, split};
     };
     const std::int64_t tiles128 = m_tiles * n128, pairs = (m_tiles + 1) / 2 * n256;
-    if (tiles128 <= sms / 2) offer(kTile128x2, kSmall.fixed + 4, kSmall.per_block, tiles128, 2, resident_clusters<128, kEpi, 1, 2>());
-    if (pairs <= sms / 4) offer(kTilePairs2, kPair.fixed + 4, kPair.per_block, pairs, 2, resident_clusters<256, kEpi, 2, 2>());
-    if (pairs <= sms / 8) offer(kTilePairs4, kPair.fixed + 12, kPair.per_block, pairs, 4, resident_clusters<256, kEpi, 2, 4>());
+    if (tiles128 <= sms / 2) offer(B2_TILE_128x128, kSmall.fixed + 4, kSmall.per_block, tiles128, 2, resident_clusters<128, kEpi, 1, 2>());
+    if (pairs <= sms / 4) offer(B2_TILE_2CTA_256x256, kPair.fixed + 4, kPair.per_block, pairs, 2, resident_clusters<256, kEpi, 2, 2>());
+    if (pairs <= sms / 8) offer(B2_TILE_2CTA_256x256, kPair.fixed + 12, kPair.per_block, pairs, 4, resident_clusters<256, kEpi, 2, 4>());
   }
   return best;
 }
 
 template <Epi kEpi>
 int dispatch(const char* op, const b2_int8_operands* a, const GemmParams& p, cudaStream_t stream, int tile) {
+  const TileChoice t = tile != B2_TILE_AUTO ? TileChoice{tile, 1} : pick_tile_int8<kEpi>(p);
+  const bool pair = t.tile == B2_TILE_2CTA_256x256;
   if constexpr (kEpi == Epi::kSituGlu) {
-    const int t = tile != B2_TILE_AUTO ? tile : pick_tile_int8<kEpi>(p);
-    return t == B2_TILE_2CTA_256x256 ? launch_kernel<256, kEpi, 2>(op, a, p, stream) : launch_kernel<256, kEpi, 1>(op, a, p, stream);
+    return pair ? launch_kernel<256, kEpi, 2>(op, a, p, stream) : launch_kernel<256, kEpi, 1>(op, a, p, stream);
   } else {
-    const int t = tile != B2_TILE_AUTO ? tile : pick_tile_int8<kEpi>(p);
-    if (t == B2_TILE_2CTA_256x256) return launch_kernel<256, kEpi, 2>(op, a, p, stream);
     if constexpr (kEpi != Epi::kAcc) {
-      if (t == kTilePairs2) return launch_kernel<256, kEpi, 2, false, 2>(op, a, p, stream);
-      if (t == kTilePairs4) return launch_kernel<256, kEpi, 2, false, 4>(op, a, p, stream);
-      if (t == kTile128x2) return launch_kernel<128, kEpi, 1, false, 2>(op, a, p, stream);
+      if (t.split == 4) return launch_kernel<256, kEpi, 2, false, 4>(op, a, p, stream);
+      if (t.split == 2) return pair ? launch_kernel<256, kEpi, 2, false, 2>(op, a, p, stream) : launch_kernel<128, kEpi, 1, false, 2>(op, a, p, stream);
     }
-    return t == B2_TILE_128x256 ? launch_kernel<256, kEpi, 1>(op, a, p, stream) : launch_kernel<128, kEpi, 1>(op, a, p, stream);
+    if (pair) return launch_kernel<256, kEpi, 2>(op, a, p, stream);
+    return t.tile == B2_TILE_128x256 ? launch_kernel<256, kEpi, 1>(op, a, p, stream) : launch_kernel<128, kEpi, 1>(op, a, p, stream);
   }
 }
 

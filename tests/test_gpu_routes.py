@@ -38,6 +38,26 @@ def test_gemm_tiles_that_share_k_give_the_bits_of_whole_tiles(ops, m, n, k):
     assert ops.kernel_status() == (0, 0)
 
 
+@pytest.mark.parametrize("tile", [-1, 4, 16, 17, 18])
+def test_gemm_tile_values_outside_the_enum_run_whole_tiles(ops, tile):
+    """A tile argument names a shape and never a split of K, which with as few K blocks as here would leave CTAs without any:
+    every value that the enum does not have runs 128 x 128 tiles."""
+    m, n = 200, 264
+    for k in (16, 128, 384):
+        g = _gen(k)
+        x = torch.randint(-127, 128, (m, k), dtype=torch.int8, device="cuda", generator=g)
+        w = torch.randint(-127, 128, (n, k), dtype=torch.int8, device="cuda", generator=g)
+        xs, ws = torch.rand(m, device="cuda", generator=g) * 1e-3, torch.rand(n, device="cuda", generator=g) * 1e-3
+        gate, res = torch.randn(n, device="cuda", generator=g).bfloat16(), torch.randn((m, n), device="cuda", generator=g).bfloat16()
+        got, want = [], []
+        for t, to in ((tile, got), (ops.TILE_128x128, want)):
+            to += [ops.int8_gemm(x, xs, w, ws, tile=t), ops.int8_gemm_chunked(x, xs, w, ws, 88, tile=t), res.clone()]
+            ops.int8_gemm_gated_residual(x, xs, w, ws, gate, to[-1], tile=t)
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    assert ops.kernel_status() == (0, 0)
+
+
 @pytest.mark.parametrize("lens", [[1], [33], [64], [65], [297], [512], [320, 266], [17, 0, 512], [100, 448, 3, 64, 449]])
 def test_prepass_of_short_sequences_in_one_launch(ops, lens):
     """max_seqlen up to 512: the pre-pass is one launch. The same call with a larger max_seqlen takes the separate kernels."""
