@@ -1,6 +1,6 @@
 // SageAttention-style 8-bit attention for sm_100a, plus the MOSS QK-norm + RoPE and RoPE-table kernels that feed it.
 //
-//   pre-pass (HBM-bound, 128-bit accesses; all of it in one launch for sequences of up to 512 tokens)
+//   pre-pass (HBM-bound, 128-bit accesses; all of it in one launch for a few sequences of up to 512 tokens)
 //     prologue   (fused QK-norm + RoPE only) per (32 tokens, head): RMS-norm + RoPE of q and k, k written back,
 //                Q quantised
 //     stats      per (512-key chunk, head, sequence): partial per-channel K sums and V |max| in a fixed order
@@ -1555,6 +1555,20 @@ struct ScoreDump {
   int seq = 0, head = 0, tile = 0;
 };
 
+// When the one-launch pre-pass is the faster one. It has a CTA for every 64 rows up to max_seqlen, with or without tokens, that
+// stays for the whole chain of steps: by the CTAs per SM (two fit; clusters of eight reach 1.73) and the share of their rows
+// that hold tokens. Measured against the four launches (24, 12, 8 or 4 heads, us):
+//   to 0.65 per SM  1 x 20 of 512 8.0 -> 6.6, 1 x 100 8.8 -> 8.3, 1 x 512 (12 heads) 17.1 -> 8.4
+//   to 1.85         2 x 297 16.5 -> 11.6, 1 x 158 of 428 (0.35) 10.8 -> 10.9, 1 x 102 of 360 (0.27) 9.8 -> 10.5
+//   to 2.6          2 x 494 of 504 (0.96) 22.5 -> 20.4, 3 x 284 (0.89) 18.6 -> 18.0, 2 x 392 of 413 (0.89) 20.3 -> 20.5,
+//                   3 x 230 of 281 (0.73) 17.0 -> 17.6, 2 x 20 of 512 (0.04) 8.9 -> 14.2
+//   beyond          9 x 345 of 363 (0.92) 20.8 -> 21.8, 8 x 512 52 -> 69, 32 x 100 of 512 68 -> 201
+bool short_prepass_pays(std::int64_t tokens, int batch, std::int64_t heads, int k_blocks) {
+  const double rows = 64.0 * k_blocks * batch, share = static_cast<double>(tokens) / rows;
+  const double per_sm = rows / 64.0 * static_cast<double>(heads) / sm_count();
+  return per_sm <= 0.65 || (per_sm <= 1.85 && share >= 0.35) || (per_sm <= 2.6 && share >= 0.9);
+}
+
 int attention_impl(const char* op, const b2_attention_options* o, const b2_view3* q, const b2_view3* k, const b2_view3* v,
                    const b2_view3* out, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int batch,
                    int max_seqlen, float scale, void* workspace, size_t workspace_bytes, void* stream,
@@ -1647,7 +1661,8 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
     p.norm_factor = static_cast<float>(norm_rows) / static_cast<float>(norm_rows * kHeadDim);
   }
   const unsigned h = static_cast<unsigned>(heads);
-  if (norm_rope != nullptr && max_seqlen <= kStatsChunk && !slots && p.all_rows == 0 && cu_seqlens_q == cu_seqlens_k) {
+  if (norm_rope != nullptr && max_seqlen <= kStatsChunk && !slots && p.all_rows == 0 && cu_seqlens_q == cu_seqlens_k &&
+      short_prepass_pays(total_q, batch, heads, l.k_blocks)) {
     // Sequences of one statistics chunk whose rows are all their own.
     if (const int rc = enqueue(op, short_prepass_kernel, dim3(l.k_blocks, h, batch), 512, 0, st, l.k_blocks, p)) return rc;
   } else {

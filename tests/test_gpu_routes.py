@@ -18,6 +18,26 @@ def _gen(seed):
     return torch.Generator("cuda").manual_seed(seed)
 
 
+def _kernels(call):
+    """The (mangled) names of the kernels that a call launches, in order of capture."""
+    from cuda.bindings import driver as cu
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+
+    def ok(r):
+        assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+        return r[1:]
+    handle = cu.CUgraph(graph.raw_cuda_graph())
+    names = []
+    for node in ok(cu.cuGraphGetNodes(handle, ok(cu.cuGraphGetNodes(handle, 0))[1]))[0]:
+        if ok(cu.cuGraphNodeGetType(node))[0] == cu.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(cu.cuGraphKernelNodeGetParams(node))[0]
+            name = cu.cuFuncGetName(params.func) if int(params.func) else cu.cuKernelGetName(params.kern)
+            names.append(ok(name)[0].decode())
+    return names
+
+
 @pytest.mark.parametrize("m", [1, 127, 256, 257, 297, 384, 512])
 @pytest.mark.parametrize("n,k", [(64, 512), (1000, 528), (3072, 3072), (3064, 8192)])
 def test_gemm_tiles_that_share_k_give_the_bits_of_whole_tiles(ops, m, n, k):
@@ -60,7 +80,8 @@ def test_gemm_tile_values_outside_the_enum_run_whole_tiles(ops, tile):
 
 @pytest.mark.parametrize("lens", [[1], [33], [64], [65], [297], [512], [320, 266], [17, 0, 512], [100, 448, 3, 64, 449]])
 def test_prepass_of_short_sequences_in_one_launch(ops, lens):
-    """max_seqlen up to 512: the pre-pass is one launch. The same call with a larger max_seqlen takes the separate kernels."""
+    """A few sequences of up to 512 tokens: the pre-pass is one launch. The same call with a larger max_seqlen takes the
+    separate kernels."""
     heads, total, batch = 3, sum(lens), len(lens)
     qkv = torch.randn((total, 3 * heads * 128), device="cuda", generator=_gen(total)).bfloat16()
     norms = [(1 + 0.1 * torch.randn(128, device="cuda", generator=_gen(i))).bfloat16() for i in (1, 2)]
@@ -72,15 +93,35 @@ def test_prepass_of_short_sequences_in_one_launch(ops, lens):
         q, k, v = (x[:, i * heads * 128:(i + 1) * heads * 128].unflatten(1, (heads, 128)) for i in range(3))
         l = ops.attention_q8_layout(total, total, batch, longest, heads)
         ws = torch.full((l.total,), 0x55, dtype=torch.uint8, device="cuda")
-        ops.attention_q8_preprocess(q, k, v, cu, cu, longest, workspace=ws, norm_rope=(norms[0], norms[1], table))
+        call = lambda: ops.attention_q8_preprocess(q, k, v, cu, cu, longest, workspace=ws, norm_rope=(norms[0], norms[1], table))
+        call()
         cut = lambda at, *shape: ws[at:at + int(np.prod(shape))].view(*shape).clone()
         rows = [cut(at, total * heads, 128) for at in (l.q_i8, l.k_i8, l.v8)]
         stats = [cut(at, batch * heads, 512) for at in (l.k_mean, l.v_scale, l.v_recp)]
         qs, ks = cut(l.q_scale, batch * heads, 4 * l.q_blocks), cut(l.k_scale, batch * heads, 4 * l.k_blocks)
         n = (max(lens) + 127) // 128 * 16, (max(lens) + 63) // 64 * 4
         got.append([x.view(torch.int16), *rows, *stats, qs[:, :n[0]], ks[:, :n[1]]])
+        names = _kernels(call)
+        assert len(names) == (4 if longest > 512 else 1) and ("short_prepass" in names[0]) == (longest <= 512), names
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("heads,lens,longest,one", [(3, [20], 512, True), (24, [297, 290], 297, True), (24, [494, 489], 504, True),
+                                                    (24, [20], 512, False), (24, [20, 20], 512, False), (12, [140, 130], 512, False),
+                                                    (24, [512] * 3, 512, False), (4, [100] * 32, 512, False), (1, [7] * 60, 512, False)])
+def test_prepass_in_one_launch_only_where_it_is_the_faster(ops, heads, lens, longest, one):
+    """A CTA for every 64 rows up to max_seqlen: many sequences, or a max_seqlen far above their lengths, take the separate
+    kernels, which look at an empty block once and leave."""
+    total = sum(lens)
+    qkv = torch.randn((total, 3 * heads * 128), device="cuda", generator=_gen(total)).bfloat16()
+    q, k, v = (qkv[:, i * heads * 128:(i + 1) * heads * 128].unflatten(1, (heads, 128)) for i in range(3))
+    norm = torch.ones(128, device="cuda").bfloat16()
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    ws = torch.empty(ops.attention_q8_workspace_bytes(total, total, len(lens), longest, heads), dtype=torch.uint8, device="cuda")
+    table = ops.moss_rope_table(1, 1, total - 1)
+    names = _kernels(lambda: ops.attention_q8_preprocess(q, k, v, cu, cu, longest, workspace=ws, norm_rope=(norm, norm, table)))
+    assert len(names) == (1 if one else 4), names
 
 
 @pytest.mark.parametrize("lens,keys", [([300, 64, 700, 129], None), ([1, 0, 257, 40], [513, 70, 64, 900]), ([130] + [40] * 31, None), ([200] + [33] * 33, None)])
