@@ -993,8 +993,9 @@ __device__ __forceinline__ void umma_bf16(std::uint32_t d_tmem, std::uint64_t a_
 }
 
 // Which (query tile, head, sequence) a CTA works on, and where the sequence's queries and keys lie. kByLength: a flat grid
-// instead of (tiles, heads, sequences), for 2 to 32 sequences (a lane each): longest sequence first, by keys and then by
-// index, so that the short ones fill the last round; ids without a tile come last. See the launch for when.
+// of as many ids as there can be tiles instead of (tiles, heads, sequences), for 2 to 32 sequences (a lane each): longest
+// sequence first, by keys and then by index, so that the short ones fill the last round; ids without a tile come last. See the
+// launch for when.
 // Called by whole warps; false: no tile.
 template <bool kByLength>
 struct TileOfCta {
@@ -1714,17 +1715,21 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
 #endif
   // Longest sequence first where lengths differ much, i.e. where the keys are well below batch x the longest: in batch order
   // sequences of 1039, 777, 2500 and 64 keys left the 480 CTAs of the longest for the end, with a thousand empty ones among
-  // them (121 us; by length 107). Of nearly equal lengths it gains nothing, and finding the tile costs each CTA some loads and
-  // shuffles (1165 + 1034 + 1165 keys: 70 us, by length 71).
+  // them (121 us; by length 107). Of nearly equal lengths it gains little, and finding the tile costs each CTA some loads and
+  // shuffles (1165 + 1034 + 1165 keys: 70 us, by length 71). Where few tiles make it useless it costs up to 0.7 us (700 + 420
+  // keys), but it also keeps the empty CTAs of a generous max_seqlen out from between the full ones (4 x 1000 keys, 4 heads,
+  // max_seqlen 4000: 40 us, by length 36). The flat grid has no more CTAs than the query rows can fill tiles: with one for every
+  // tile up to max_seqlen the search of the empty ones took 32 x 100 keys from 61 to 74 us at a max_seqlen of 1000 and from 468
+  // to 840 at 16384.
+  const std::int64_t most_tiles = std::min<std::int64_t>(static_cast<std::int64_t>(a.q_tiles) * batch, (total_q + (kTileQ - 1LL) * batch) / kTileQ) * heads;
   const bool by_length = dump == nullptr && batch > 1 && batch <= 32 && 100 * total_k < 85LL * batch * max_seqlen;
   const auto kernel = dump != nullptr ? attention_kernel<true, false> : by_length ? attention_kernel<false, true> : attention_kernel<false, false>;
   if (const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
       e != cudaSuccess) {
     return fail_cuda(op, e);
   }
-  // (2^31 tiles, more than a flat grid holds, want a workspace of 500 GB.)
-  const dim3 grid = by_length ? dim3(static_cast<unsigned>(static_cast<std::int64_t>(a.q_tiles) * heads * batch))
-                              : dim3(a.q_tiles, static_cast<unsigned>(heads), batch);
+  // (By length fewer than 2^22 tiles: rows x heads is below 2^25, and 32 x 65535 more that are not full.)
+  const dim3 grid = by_length ? dim3(static_cast<unsigned>(most_tiles)) : dim3(a.q_tiles, static_cast<unsigned>(heads), batch);
   return enqueue(op, kernel, grid, kAttnThreads, kAttnSmem, st, 1, map_q, map_k, map_v, a);
 }
 }  // namespace

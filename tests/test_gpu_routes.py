@@ -124,15 +124,21 @@ def test_prepass_in_one_launch_only_where_it_is_the_faster(ops, heads, lens, lon
     assert len(names) == (1 if one else 4), names
 
 
-@pytest.mark.parametrize("lens,keys", [([300, 64, 700, 129], None), ([1, 0, 257, 40], [513, 70, 64, 900]), ([130] + [40] * 31, None), ([200] + [33] * 33, None)])
-def test_attention_of_a_batch_is_that_of_its_sequences(ops, lens, keys):
-    """Sequences of different lengths are handed out longest first up to 32 of them, in batch order beyond."""
-    heads, keys = 2, keys or lens
+@pytest.mark.parametrize("heads,lens,keys,longest,by_length", [
+    (64, [300, 64, 700, 129], None, 700, True), (64, [1, 0, 257, 40], [513, 70, 64, 900], 900, True), (12, [130] + [40] * 31, None, 130, True),
+    (12, [129] * 31, None, 16384, True), (64, [128, 1, 129, 1], None, 5000, True), (64, [1] * 32, None, 512, True), (64, [0, 128, 0, 513], None, 513, True),
+    (64, [200] + [33] * 33, None, 200, False), (3, [300, 64, 700, 129], None, 700, True), (1, [130, 2], None, 4096, True), (64, [300, 290], None, 300, False)])
+def test_attention_of_a_batch_is_that_of_its_sequences(ops, heads, lens, keys, longest, by_length):
+    """Sequences of different lengths are handed out longest first, up to 32 of them; else in batch order. The flat grid has to
+    reach the last tile whatever the lengths leave of each tile."""
+    keys = keys or lens
     q = torch.randn((sum(lens), heads, 128), device="cuda", generator=_gen(5)).bfloat16()
     k, v = (torch.randn((sum(keys), heads, 128), device="cuda", generator=_gen(s)).bfloat16() for s in (6, 7))
     cu = lambda n: torch.tensor(np.concatenate([[0], np.cumsum(n)]), dtype=torch.int32, device="cuda")
-    out, want = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
-    ops.attention_q8(q, k, v, out, cu(lens), cu(keys), max(lens + keys), ops.SM_SCALE)
+    out, want, cq, ck = torch.full_like(q, 7.0), torch.full_like(q, 7.0), cu(lens), cu(keys)
+    ws = torch.empty(ops.attention_q8_workspace_bytes(sum(lens), sum(keys), len(lens), longest, heads), dtype=torch.uint8, device="cuda")
+    call = lambda: ops.attention_q8(q, k, v, out, cq, ck, longest, ops.SM_SCALE, workspace=ws)
+    call()
     a = b = 0
     for n, m in zip(lens, keys):
         if n > 0:
@@ -140,3 +146,4 @@ def test_attention_of_a_batch_is_that_of_its_sequences(ops, lens, keys):
         a, b = a + n, b + m
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
     assert ops.kernel_status() == (0, 0)
+    assert ("ILb0ELb1E" in _kernels(call)[-1]) == by_length, _kernels(call)[-1]
