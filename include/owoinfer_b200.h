@@ -666,8 +666,9 @@ int b2_kernel_status_clear(void);
 /* Test hook of the bounded waits. wait_limit_ns != 0 sets how long a wait inside the GEMM kernel may last on the current
  * device (default 200 ms; the attention kernel's limit is fixed at 200 ms). skip_gemm_stage != 0 makes the TMA warp of
  * every GEMM CTA leave out the loads of the last K block of its first tile: that stage's barrier then never completes,
- * the waits run out after the limit, every CTA raises the status word, drains, frees its tensor memory and returns (the
- * output of that launch is garbage, nothing faults or hangs). Call again with (0-or-limit, 0) to switch it off.
+ * the waits run out after the limit, every CTA raises the status word, drains, frees its tensor memory and returns (a tile
+ * whose K range was not summed in full is not stored, nothing faults or hangs). 2 does so only in the CTAs with the first
+ * part of K where a cluster shares a tile's K range. Call again with (0-or-limit, 0) to switch it off.
  * No counterpart in the reference. */
 int b2_debug_bounded_wait(uint64_t wait_limit_ns, int skip_gemm_stage);
 

@@ -360,6 +360,9 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void st_cluster_v4(std::uint32_t cluster_addr, std::uint32_t x, std::uint32_t y, std::uint32_t z, std::uint32_t w) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+__device__ __forceinline__ void st_cluster_u32(std::uint32_t cluster_addr, std::uint32_t x) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(x) : "memory");
+}
 // Arrive on an mbarrier given by its shared::cluster address (own or peer CTA).
 __device__ __forceinline__ void mbar_arrive_cluster(std::uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");

@@ -103,7 +103,8 @@ __device__ int g_gemm_status = 0;  // set to 1 by a CTA whose bounded wait expir
 // notice it.
 __device__ unsigned long long g_gemm_wait_limit_ns = 200000000ull;
 // Test hook: 1 = the TMA warp of every CTA leaves out the loads of the last K block of its first tile, so that the
-// stage's barrier never completes and the bounded waits run out.
+// stage's barrier never completes and the bounded waits run out; 2 = where a cluster shares a tile's K range, only the CTA
+// (pair) with the first part of it does.
 __device__ int g_gemm_test_skip_stage = 0;
 
 __device__ __forceinline__ std::uint64_t global_ns() {
@@ -210,7 +211,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   // scale. 4 KB, filled once per CTA.
   __shared__ __align__(16) uint4 s_lut[kW4 ? 256 : 1];
   __shared__ std::uint32_t s_tmem_base;
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_lost;  // s_lost: a CTA that this tile's K range is shared with has nothing to hand over
   // Per epilogue warp: w_scale, bias, gate of its 128 columns (SiTU-GLU: w_scale of its 32 hidden and 32 gate columns).
   constexpr int kEpiWarps = epi_warps(kEpi, kBN, kW4), kVecFloats = kEpi == Epi::kSituGlu ? 64 * (16 / epi_warps(kEpi, kBN, kW4)) : 384;
   __shared__ __align__(16) float s_vec[kEpiWarps][kVecFloats];
@@ -237,7 +238,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       mbar_init(smem_u32(&s_tmem_full[i]), 1);
       mbar_init(smem_u32(&s_tmem_empty[i]), kEpiWarps * kCtas);
     }
-    s_abort = 0;
+    s_abort = 0, s_lost = 0;
     fence_mbar_init();
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
@@ -312,7 +313,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int row_a = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM;
         int row_b0, row_b1;
         b_rows(nt, row_b0, row_b1);
-        const bool skip_last = g_gemm_test_skip_stage != 0 && tile == tile0;
+        const bool skip_last = g_gemm_test_skip_stage != 0 && tile == tile0 && (g_gemm_test_skip_stage == 1 || split == 0);
         for (int kb = kb_first; kb < k_blocks; ++kb, ++it) {
           const int s = static_cast<int>(it % kStages);
           const std::uint32_t ph = (it / kStages) & 1u;
@@ -596,9 +597,13 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if constexpr (kSplit > 1) {
         // Every CTA of the cluster is past its last MMA: the rings are free. Accumulator columns of the other splits go to
         // their CTA of the same rows, 16 bytes per lane side by side, where the same lane of that CTA finds them.
+        // A CTA whose wait ran out has nothing to hand over, and without its part no sum of the tile is whole: it tells every
+        // CTA of the cluster between the two barriers, and none stores anything.
         landed = !__any_sync(0xffffffffu, !landed);
         cluster_sync_all();
-        if (landed) {
+        if (!landed) {
+          if (lane < kCluster) st_cluster_u32(map_to_cta(smem_u32(&s_lost), static_cast<std::uint32_t>(lane)), 1u);
+        } else {
 #pragma unroll 1
           for (int unit = col_half; unit < kBN / 64; unit += 2) {
             const int owner = unit / kOwnUnits;
@@ -617,7 +622,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           }
         }
         cluster_sync_all();
-        if (!landed || !has_part) break;
+        if (s_lost != 0 || !has_part) break;
       }
       const int row = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM + quarter * 32 + lane;
       const bool row_ok = row < p.m;

@@ -303,8 +303,8 @@ def kernel_status_clear():
     check(_lib.lib().b2_kernel_status_clear())
 
 
-def debug_bounded_wait(wait_limit_ns: int, skip_gemm_stage: bool):
-    check(_lib.lib().b2_debug_bounded_wait(C.c_uint64(wait_limit_ns), C.c_int(1 if skip_gemm_stage else 0)))
+def debug_bounded_wait(wait_limit_ns: int, skip_gemm_stage: int):
+    check(_lib.lib().b2_debug_bounded_wait(C.c_uint64(wait_limit_ns), C.c_int(int(skip_gemm_stage))))
 
 
 # ------------------------------------------------------------------------------------------------ block / step

@@ -1,4 +1,6 @@
 """Routes that a rule on sizes picks, against the general route of the same call: the same bits."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -55,6 +57,41 @@ def test_gemm_tiles_that_share_k_give_the_bits_of_whole_tiles(ops, m, n, k):
     ops.int8_gemm_gated_residual(x, xs, w, ws, gate, res)
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     assert torch.equal(res.view(torch.int16), want_res.view(torch.int16))
+    assert ops.kernel_status() == (0, 0)
+
+
+def _gemm_route(call):
+    """(tile columns, CTAs of a tile, CTAs or pairs that share its K range) of the one INT8 GEMM kernel that a call launches."""
+    name, = _kernels(call)
+    return tuple(int(v) for v in re.search(r"int8_gemm_kernelILi(\d+)E.*?ELi(\d)ELb0ELi(\d)E", name).groups())
+
+
+@pytest.mark.parametrize("skip", [1, 2])
+@pytest.mark.parametrize("m,n,k,route", [(300, 1024, 8192, (128, 1, 2)), (400, 3064, 8208, (256, 2, 2)), (129, 2056, 16400, (256, 2, 4))])
+def test_bounded_wait_of_a_shared_tile_stores_nothing(ops, m, n, k, route, skip):
+    """One CTA's wait (skip 2: that of the first part of K only) runs out: no CTA of its cluster has the whole sum, so none stores,
+    neither a result nor into the residual stream. The status word is raised and the next call is right."""
+    g = _gen(m + n + k)
+    x = torch.randint(-127, 128, (m, k), dtype=torch.int8, device="cuda", generator=g)
+    w = torch.randint(-127, 128, (n, k), dtype=torch.int8, device="cuda", generator=g)
+    xs, ws = torch.rand(m, device="cuda", generator=g) * 1e-3, torch.rand(n, device="cuda", generator=g) * 1e-3
+    gate, res = torch.randn(n, device="cuda", generator=g).bfloat16(), torch.randn((m, n), device="cuda", generator=g).bfloat16()
+    out, got_res = torch.full((m, n), 7.0, dtype=torch.bfloat16, device="cuda"), res.clone()
+    assert _gemm_route(lambda: ops.int8_gemm(x, xs, w, ws, out=out)) == route
+    torch.cuda.synchronize()
+    assert ops.kernel_status() == (0, 0)
+    ops.debug_bounded_wait(2_000_000, skip)
+    try:
+        ops.int8_gemm(x, xs, w, ws, out=out)
+        ops.int8_gemm_gated_residual(x, xs, w, ws, gate, got_res)
+        torch.cuda.synchronize()
+        assert ops.kernel_status() == (1, 0)
+    finally:
+        ops.debug_bounded_wait(200_000_000, 0)
+        ops.kernel_status_clear()
+    assert torch.equal(out, torch.full_like(out, 7.0)) and torch.equal(got_res, res)
+    ops.int8_gemm(x, xs, w, ws, out=out)
+    assert torch.equal(out.view(torch.int16), ops.int8_gemm(x, xs, w, ws, tile=ops.TILE_128x128).view(torch.int16))
     assert ops.kernel_status() == (0, 0)
 
 
