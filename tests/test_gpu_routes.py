@@ -66,6 +66,38 @@ def _gemm_route(call):
     return tuple(int(v) for v in re.search(r"int8_gemm_kernelILi(\d+)E.*?ELi(\d)ELb0ELi(\d)E", name).groups())
 
 
+# Both ends of a tile's rows, columns that end inside a 64-column unit, K blocks that the CTAs of a cluster cannot share evenly (65,
+# 97, 17 of them), and a last K block that is not full.
+SHARED_K = [(1, 3064, 8208, (128, 1, 2)), (257, 3072, 3088, (128, 1, 2)), (384, 3064, 8208, (128, 1, 2)), (100, 1000, 2064, (128, 1, 2)),
+            (128, 9216, 3072, (128, 1, 2)), (385, 3064, 8208, (256, 2, 2)), (400, 3064, 12304, (256, 2, 2)), (512, 3072, 8208, (256, 2, 2)),
+            (1, 3064, 12288, (256, 2, 4)), (129, 2056, 16400, (256, 2, 4)), (256, 3072, 12304, (256, 2, 4))]
+
+
+@pytest.mark.parametrize("m,n,k,route", SHARED_K)
+def test_each_way_of_sharing_k_gives_the_bits_of_whole_tiles(ops, m, n, k, route):
+    """The three cluster shapes that AUTO takes for few rows, by the kernel that is launched: plain, column-chunked and
+    gated-residual outputs against whole 128 x 128 tiles."""
+    g = _gen(m * 7 + n + k)
+    x = torch.randint(-127, 128, (m, k), dtype=torch.int8, device="cuda", generator=g)
+    w = torch.randint(-127, 128, (n, k), dtype=torch.int8, device="cuda", generator=g)
+    xs, ws = torch.rand(m, device="cuda", generator=g) * 1e-3, torch.rand(n, device="cuda", generator=g) * 1e-3
+    bias, gate = (torch.randn(n, device="cuda", generator=g).bfloat16() for _ in range(2))
+    res = torch.randn((m, n), device="cuda", generator=g).bfloat16()
+    want, want_res = ops.int8_gemm(x, xs, w, ws, bias, tile=ops.TILE_128x128), res.clone()
+    ops.int8_gemm_gated_residual(x, xs, w, ws, gate, want_res, tile=ops.TILE_128x128)
+    chunk = n // 8 if n % 64 == 0 else n
+    got, chunks, out_res = ops.int8_gemm(x, xs, w, ws, bias), ops.int8_gemm_chunked(x, xs, w, ws, chunk, bias=bias), res.clone()
+    ops.int8_gemm_gated_residual(x, xs, w, ws, gate, out_res)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert torch.equal(chunks.permute(1, 0, 2).reshape(m, n).view(torch.int16), want.view(torch.int16))
+    assert torch.equal(out_res.view(torch.int16), want_res.view(torch.int16))
+    assert ops.kernel_status() == (0, 0)
+    scratch = res.clone()
+    assert _gemm_route(lambda: ops.int8_gemm(x, xs, w, ws, bias, out=got)) == route
+    assert _gemm_route(lambda: ops.int8_gemm_chunked(x, xs, w, ws, chunk, bias=bias, out=chunks)) == route
+    assert _gemm_route(lambda: ops.int8_gemm_gated_residual(x, xs, w, ws, gate, scratch)) == route
+
+
 @pytest.mark.parametrize("skip", [1, 2])
 @pytest.mark.parametrize("m,n,k,route", [(300, 1024, 8192, (128, 1, 2)), (400, 3064, 8208, (256, 2, 2)), (129, 2056, 16400, (256, 2, 4))])
 def test_bounded_wait_of_a_shared_tile_stores_nothing(ops, m, n, k, route, skip):
