@@ -25,7 +25,10 @@ def _stream() -> C.c_void_p:
     if not torch.cuda.is_initialized():
         return C.c_void_p(torch.cuda.current_stream().cuda_stream)
     # The same handle without the Stream object around it, whose making is a good part of a small call.
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    try:
+        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    except AttributeError:  # private names, which another torch may not have
+        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _ptr(t) -> C.c_void_p:

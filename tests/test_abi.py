@@ -318,3 +318,18 @@ def test_python_layer_fails_loudly_without_library(tmp_path, monkeypatch):
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "missing.so"))
     with pytest.raises(RuntimeError, match="no fallback"):
         _lib.lib()
+
+
+@pytest.mark.parametrize("gone", ["_cuda_getCurrentRawStream", "_cuda_getDevice"])
+def test_stream_without_the_private_names_of_torch(monkeypatch, gone):
+    import types
+
+    import torch
+    from owoinfer_b200 import ops
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=0x1234))
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 0x99, raising=False)
+    assert ops._stream().value == 0x99
+    monkeypatch.delattr(torch._C, gone)
+    assert ops._stream().value == 0x1234
