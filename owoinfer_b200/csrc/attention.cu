@@ -1038,11 +1038,10 @@ struct TileOfCta {
 //                 pipelined: the loads of S(u + 1) are issued right after P(u) is handed over and land during the
 //                 bookkeeping in between, and the K scale of the next sub-tile is fetched a whole pass ahead.
 //   P             e4m3, the A operand of P·V in tensor memory (64 keys = 16 columns), in the first columns of the score
-//                 buffer it came from: the next scores go there by MMAs issued behind the ones that read P. With P in shared
-//                 memory (a swizzled 16 KB tile) one pair of sub-tiles kept the shared-memory port of an SM (128 bytes a
-//                 clock: the CTAs' K/V tiles in, the MMAs' operands out, P both ways) busy for about 1120 of the 1590 clocks
-//                 it took; without P it is 860. Kernel alone at 2 x 8192 tokens: 1212 -> 1166 us (1414 TOP/s), at 20480 keys
-//                 3649 -> 3516 us, at 4096 keys 194 -> 186 us; same bits.
+//                 buffer it came from; the next scores go there once the MMAs that read P have landed. With P in shared
+//                 memory (a swizzled 16 KB tile) one pair of sub-tiles keeps the shared-memory port of an SM (128 bytes a
+//                 clock: the CTAs' K/V tiles in, the MMAs' operands out, P both ways) busy for about 1120 of its 1590 clocks;
+//                 without P it is 860.
 // kDump: the instantiation behind b2_attention_q8_debug_scores, which also stores one tile's raw integer scores.
 template <bool kDump, bool kByLength>
 __global__ void __launch_bounds__(kAttnThreads, 2)
@@ -1066,7 +1065,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
   extern __shared__ std::uint8_t smem_raw[];
   __shared__ __align__(8) std::uint64_t s_q_full, s_k_full[kKvStages], s_k_empty[kKvStages], s_v_full[kKvStages],
-      s_v_empty[kKvStages], s_step[2], s_p_full[2], s_s_ready;
+      s_v_empty[kKvStages], s_step[2], s_p_read, s_p_full[2], s_s_ready;
   __shared__ std::uint32_t s_tmem_base;
   __shared__ int s_abort;
   const std::uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -1087,6 +1086,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       mbar_init(smem_u32(&s_step[i]), 1);
       mbar_init(smem_u32(&s_p_full[i]), 4);
     }
+    mbar_init(smem_u32(&s_p_read), 1);
     mbar_init(smem_u32(&s_s_ready), 4);
     s_abort = 0;
     fence_mbar_init();
@@ -1159,11 +1159,12 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       tc_commit(smem_u32(&s_k_empty[0]));
     }
     __syncwarp();
-    // Step u, once the softmax warps have consumed S(u) and written P(u): O += P(u) · V(u), then S(u + 2), whose columns hold
-    // P(u); one completion for both. All of a step is issued in one go behind its waits: with the vote, the fence and the
-    // election once for P·V and once for the scores the warp needed 1580 clocks a step even with softmax warps that did next
-    // to nothing, now 1240 (8192 + 8192 keys: 1033 -> 893 us in that timing-only build, 1174 -> 1159 us in the product,
-    // 512 -> 497 us on peaked scores at 4378 + 4106). (By a single lane instead of the whole warp: 1216 us.)
+    // Step u, once the softmax warps have consumed S(u) and written P(u): O += P(u) · V(u), then S(u + 2) into the columns
+    // that hold P(u), then one completion for both. The scores wait for P·V to land: tcgen05.mma instructions keep their order
+    // only where accumulator and shape are the same, which these two do not share, so nothing else says that P(u) has been
+    // read by then. The wait costs 0.2 to 2.7 % of a whole call, 4 % where a CTA has an SM to itself (2048 keys, 6 heads) and up
+    // to 7.7 % on long peaked scores (16400 keys, 8 heads); P in the other score buffer, which needs no such wait but has S(u + 1)
+    // read out first, costs 2 to 8 % and up to 14 %. One election for all of a step: one for each half of it is slower by 0.2 %.
     for (int t = 0; ok && t < n_tiles; ++t) {
       const int s = t % kKvStages, s_next = (t + 1) % kKvStages;
 #pragma unroll
@@ -1188,10 +1189,17 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           const std::uint64_t dv = (s != 0 ? dv1 : dv0) + h * kHalfTile;
           umma_f8_ts(tmem_o, d_s, dv, idesc_pv, u != 0 ? 1u : 0u);
           umma_f8_ts(tmem_o, d_s + 8u, dv + 256u, idesc_pv, 1u);
-          if (more) issue_scores(d_s, (s_next != 0 ? dk1 : dk0) + h * kHalfTile);
-          tc_commit(smem_u32(&s_step[h]));
+          if (more) tc_commit(smem_u32(&s_p_read));
           if (h == 1 || u + 1 >= n_sub) tc_commit(smem_u32(&s_v_empty[s]));
-          if (more && (h == 1 || u + 3 >= n_sub)) tc_commit(smem_u32(&s_k_empty[s_next]));
+          // (Completion u. Should it never come, the step is not completed and the waits on that give up.)
+          if (!more || wait_bar(smem_u32(&s_p_read), h, abort_word)) {
+            if (more) {
+              tc_fence_after();
+              issue_scores(d_s, (s_next != 0 ? dk1 : dk0) + h * kHalfTile);
+            }
+            tc_commit(smem_u32(&s_step[h]));
+            if (more && (h == 1 || u + 3 >= n_sub)) tc_commit(smem_u32(&s_k_empty[s_next]));
+          }
         }
         __syncwarp();
         TRACE(7);

@@ -216,3 +216,25 @@ def test_attention_of_a_batch_is_that_of_its_sequences(ops, heads, lens, keys, l
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
     assert ops.kernel_status() == (0, 0)
     assert ("ILb0ELb1E" in _kernels(call)[-1]) == by_length, _kernels(call)[-1]
+
+
+@pytest.mark.parametrize("lens", [[129], [4160], [8192, 1, 3000]])
+def test_attention_does_not_depend_on_what_shares_the_sms(ops, lens):
+    """P lies where later scores go: a head's output is the same bits with two CTAs on an SM, alone, and in every one of many
+    launches (short and long pipelines, scores that make the softmax raise its reference)."""
+    heads, total = 24, sum(lens)
+    q, k, v = (torch.randn((total, heads, 128), device="cuda", generator=_gen(s)) for s in (8, 9, 10))
+    k = (k * torch.linspace(0.1, 5.0, total, device="cuda")[:, None, None]).bfloat16()
+    q, v = q.bfloat16(), v.bfloat16()
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    out, first = torch.empty_like(q), torch.empty_like(q)
+    ws = torch.empty(ops.attention_q8_workspace_bytes(total, total, len(lens), max(lens), heads), dtype=torch.uint8, device="cuda")
+    ops.attention_q8(q, k, v, first, cu, cu, max(lens), ops.SM_SCALE, workspace=ws)
+    for _ in range(20):
+        ops.attention_q8(q, k, v, out.fill_(7.0), cu, cu, max(lens), ops.SM_SCALE, workspace=ws)
+        assert torch.equal(out.view(torch.int16), first.view(torch.int16))
+    for h in (0, 11, 23):
+        one = out[:, h:h + 1].clone()
+        ops.attention_q8(q[:, h:h + 1], k[:, h:h + 1], v[:, h:h + 1], one, cu, cu, max(lens), ops.SM_SCALE)
+        assert torch.equal(one.view(torch.int16), first[:, h:h + 1].view(torch.int16))
+    assert ops.kernel_status() == (0, 0)
