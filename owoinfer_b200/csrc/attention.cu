@@ -793,6 +793,7 @@ __global__ void __launch_bounds__(512, 2) short_prepass_kernel(const PrepArgs p)
       for (int c = 0; c < ctas; ++c) a = fmaxf(a, ld_cluster_f32(map_to_cta(smem_u32(&s_vmax[ch]), static_cast<std::uint32_t>(c))));
       const float mean = len > 0 ? rbf(s / static_cast<float>(len)) : 0.f, recp = a > 0.f ? p.v_range / a : 1.f;
       const std::int64_t at = (static_cast<std::int64_t>(b) * p.heads + h) * kHeadDim + ch;
+      p.part_sum[at] = s, p.part_amax[at] = a;  // (one chunk)
       p.k_mean[at] = mean;
       p.v_scale[at] = a > 0.f ? a / p.v_range : 1.f;
       p.v_recp[at] = recp;

@@ -176,6 +176,31 @@ def test_prepass_of_short_sequences_in_one_launch(ops, lens):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("lens", [[1], [297], [17, 0, 512], [100, 448, 3, 64, 449]])
+def test_prepass_in_one_launch_leaves_the_whole_layout(ops, lens):
+    """Every area of the documented workspace layout that the separate kernels fill: the partial sums and maxima too, which with
+    sequences of one chunk are the channel's sum and maximum."""
+    heads, total, batch = 3, sum(lens), len(lens)
+    qkv = torch.randn((total, 3 * heads * 128), device="cuda", generator=_gen(total)).bfloat16()
+    norm, table = torch.ones(128, dtype=torch.bfloat16, device="cuda"), ops.moss_rope_table(1, 1, total - 1)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    got = []
+    for longest in (max(lens), 513):  # one launch; the separate kernels, whose second chunk is empty
+        q, k, v = (qkv.clone()[:, i * heads * 128:(i + 1) * heads * 128].unflatten(1, (heads, 128)) for i in range(3))
+        l = ops.attention_q8_layout(total, total, batch, longest, heads)
+        ws = torch.full((l.total,), 0x55, dtype=torch.uint8, device="cuda")
+        call = lambda: ops.attention_q8_preprocess(q, k, v, cu, cu, longest, workspace=ws, norm_rope=(norm, norm, table))
+        assert len(_kernels(call)) == (1 if longest <= 512 else 4)
+        q, k, v = (qkv.clone()[:, i * heads * 128:(i + 1) * heads * 128].unflatten(1, (heads, 128)) for i in range(3))
+        call()
+        parts = [ws[at:at + batch * heads * l.chunks * 512].view(torch.int32).view(batch, heads, l.chunks, 128)[:, :, 0].clone()
+                 for at in (l.part_sum, l.part_amax)]
+        assert l.chunks == (1 if longest <= 512 else 2)
+        got.append(parts)
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("heads,lens,longest,one", [(3, [20], 512, True), (24, [297, 290], 297, True), (24, [494, 489], 504, True),
                                                     (24, [20], 512, False), (24, [20, 20], 512, False), (12, [140, 130], 512, False),
                                                     (24, [512] * 3, 512, False), (4, [100] * 32, 512, False), (1, [7] * 60, 512, False)])
