@@ -102,9 +102,10 @@ __device__ int g_gemm_status = 0;  // set to 1 by a CTA whose bounded wait expir
 // before this one first, so the longest wait of a healthy launch is one K loop, tens of microseconds); an operator does not
 // notice it.
 __device__ unsigned long long g_gemm_wait_limit_ns = 200000000ull;
-// Test hook: 1 = the TMA warp of every CTA leaves out the loads of the last K block of its first tile, so that the
-// stage's barrier never completes and the bounded waits run out; 2 = where a cluster shares a tile's K range, only the CTA
-// (pair) with the first part of it does.
+// Test hook: not 0 = the TMA warp of every CTA leaves out the loads of the last K block of its first tile, so that the
+// stage's barrier never completes and the bounded waits run out. Where a cluster shares a tile's K range: of the CTAs (pairs)
+// with the first this many parts of it. (Read once per tile, in a form that the compiler keeps out of the loop over K blocks: a
+// test in there costs 5 % of a GEMM bound by the tensor cores.)
 __device__ int g_gemm_test_skip_stage = 0;
 
 __device__ __forceinline__ std::uint64_t global_ns() {
@@ -313,7 +314,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int row_a = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM;
         int row_b0, row_b1;
         b_rows(nt, row_b0, row_b1);
-        const bool skip_last = g_gemm_test_skip_stage != 0 && tile == tile0 && (g_gemm_test_skip_stage == 1 || split == 0);
+        const bool skip_last = (kSplit == 1 ? g_gemm_test_skip_stage != 0 : g_gemm_test_skip_stage > split) && tile == tile0;
         for (int kb = kb_first; kb < k_blocks; ++kb, ++it) {
           const int s = static_cast<int>(it % kStages);
           const std::uint32_t ph = (it / kStages) & 1u;
@@ -1179,7 +1180,8 @@ int gemm_debug_set(unsigned long long wait_limit_ns, int skip_stage) {
       return fail_cuda("debug_bounded_wait", e);
     }
   }
-  const cudaError_t e = cudaMemcpyToSymbol(g_gemm_test_skip_stage, &skip_stage, sizeof(int));
+  const int parts = skip_stage == 2 ? 1 : skip_stage != 0 ? 4 : 0;
+  const cudaError_t e = cudaMemcpyToSymbol(g_gemm_test_skip_stage, &parts, sizeof(int));
   return e == cudaSuccess ? B2_OK : fail_cuda("debug_bounded_wait", e);
 }
 
