@@ -201,6 +201,37 @@ def test_prepass_in_one_launch_leaves_the_whole_layout(ops, lens):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("layout", ["apart", "heads first", "padded rows", "head gaps"])
+def test_prepass_in_one_launch_for_other_strides(ops, layout):
+    """q, k and v in tensors of their own, with the heads outermost, with rows or heads that leave a gap, a table whose rows leave
+    one, and values in another layout than the keys: one launch and the separate kernels give the same."""
+    heads, lens = 4, [65, 0, 300, 1]
+    total, batch = sum(lens), len(lens)
+    shape = {"apart": (total, heads, 128), "heads first": (heads, total, 128), "padded rows": (total, heads * 128 + 40), "head gaps": (total, heads, 136)}[layout]
+    view = {"apart": lambda t: t, "heads first": lambda t: t.transpose(0, 1), "padded rows": lambda t: t[:, :heads * 128].unflatten(1, (heads, 128)),
+            "head gaps": lambda t: t[:, :, :128]}[layout]
+    norms = [(1 + 0.1 * torch.randn(128, device="cuda", generator=_gen(i))).bfloat16() for i in (1, 2)]
+    table = torch.cat([ops.moss_rope_table(1, 1, n - 1) for n in lens if n > 0])
+    wide = torch.zeros((total, table.shape[1] + 64), dtype=torch.bfloat16, device="cuda")
+    wide[:, :table.shape[1]] = table
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    got = []
+    for longest in (300, 513):
+        tq, tk = (torch.randn(shape, device="cuda", generator=_gen(i)).bfloat16() for i in (3, 4))
+        q, k, v = view(tq), view(tk), torch.randn((heads, total, 128), device="cuda", generator=_gen(5)).bfloat16().transpose(0, 1)
+        l = ops.attention_q8_layout(total, total, batch, longest, heads)
+        ws = torch.full((l.total,), 0x55, dtype=torch.uint8, device="cuda")
+        call = lambda: ops.attention_q8_preprocess(q, k, v, cu, cu, longest, workspace=ws, norm_rope=(norms[0], norms[1], wide[:, :table.shape[1]]))
+        assert len(_kernels(call)) == (1 if longest <= 512 else 4)
+        call()
+        cut = lambda at, *shape: ws[at:at + int(np.prod(shape))].view(*shape).clone()
+        scales = [cut(at, batch * heads, 4 * n)[:, :4 * m] for at, n, m in ((l.q_scale, l.q_blocks, 12), (l.k_scale, l.k_blocks, 5))]
+        got.append([tk.view(torch.int16), *(cut(at, total * heads, 128) for at in (l.q_i8, l.k_i8, l.v8)),
+                    *(cut(at, batch * heads, 512) for at in (l.k_mean, l.v_scale, l.v_recp)), *scales])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("heads,lens,longest,one", [(3, [20], 512, True), (24, [297, 290], 297, True), (24, [494, 489], 504, True),
                                                     (24, [20], 512, False), (24, [20, 20], 512, False), (12, [140, 130], 512, False),
                                                     (24, [512] * 3, 512, False), (4, [100] * 32, 512, False), (1, [7] * 60, 512, False)])
