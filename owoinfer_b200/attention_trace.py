@@ -19,7 +19,7 @@ SOFTMAX = [(4, "loop top"), (8, "scale of the sub-tile ready"), (0, "S(u) in reg
            (9, "vote: nothing to rescale"), (2, "pass stands"), (10, "P(u) in tensor memory"), (11, "tcgen05 fence + __syncwarp"),
            (3, "arrived on p_full(u)"), (12, "S(u+1) computed, P.V(u-1) landed (s_step wait)"), (13, "loads of S(u+1) issued"),
            (14, "headroom check done")]
-MMA = [(5, "p_full(u) seen"), (7, "P.V(u) and Q.K^T(u+2) issued, step committed")]
+MMA = [(5, "p_full(u) seen"), (7, "P.V(u) landed, Q.K^T(u+2) issued, step committed")]
 
 
 def build_trace() -> str:
