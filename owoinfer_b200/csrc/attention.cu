@@ -1343,7 +1343,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (dead) break;
       TRACE(2);
       // Whether S(u + 1) is there, asked ahead of the hand-over so that the answer comes under it (usually yes: it was issued
-      // with step u - 1). 1039 + 777 + 2500 + 64 keys 104.7 -> 103.7 us, 2 x 8192 1158 -> 1154, peaked scores 497 -> 494.
+      // with step u - 1). Asked behind it the kernel takes 0.3 to 1 % longer.
       const bool next_ready = u + 1 >= n_sub || mbar_test_wait(smem_u32(&s_step[(u + 1) & 1]), ((u + 1) >> 1) & 1u);
       tmem_st_32x16(s_cols, p);
       d_run += d_tile;
@@ -1723,13 +1723,14 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   }
 #endif
   // Longest sequence first where lengths differ much, i.e. where the keys are well below batch x the longest: in batch order
-  // sequences of 1039, 777, 2500 and 64 keys left the 480 CTAs of the longest for the end, with a thousand empty ones among
+  // sequences of 1039, 777, 2500 and 64 keys leave the 480 CTAs of the longest for the end, with a thousand empty ones among
   // them (121 us; by length 107). Of nearly equal lengths it gains little, and finding the tile costs each CTA some loads and
-  // shuffles (1165 + 1034 + 1165 keys: 70 us, by length 71). Where few tiles make it useless it costs up to 0.7 us (700 + 420
-  // keys), but it also keeps the empty CTAs of a generous max_seqlen out from between the full ones (4 x 1000 keys, 4 heads,
-  // max_seqlen 4000: 40 us, by length 36). The flat grid has no more CTAs than the query rows can fill tiles: with one for every
-  // tile up to max_seqlen the search of the empty ones took 32 x 100 keys from 61 to 74 us at a max_seqlen of 1000 and from 468
-  // to 840 at 16384.
+  // shuffles. Over 256 mixes (2 to 32 sequences, the longest 300 to 3000, 6 and 24 heads) whole calls by length took, by how full
+  // batch x longest was: to 0.7 0.955 of batch order, to 0.8 0.97, to 0.86 0.99, to 0.93 0.998, above 1.005 to 1.012. (The one mix of
+  // those below the line that loses more than 3 %: 2400 + 3000 + 1800 keys, 6 heads, 86 us, by length 94.) It also keeps the
+  // empty CTAs of a generous max_seqlen out from between the full ones (4 x 1000 keys, 4 heads, max_seqlen 4000: 40 us, by length
+  // 36). The flat grid has no more CTAs than the query rows can fill tiles: with one for every tile up to max_seqlen the search of
+  // the empty ones takes 32 x 100 keys from 61 to 74 us at a max_seqlen of 1000 and from 468 to 840 at 16384.
   const std::int64_t most_tiles = std::min<std::int64_t>(static_cast<std::int64_t>(a.q_tiles) * batch, (total_q + (kTileQ - 1LL) * batch) / kTileQ) * heads;
   const bool by_length = dump == nullptr && batch > 1 && batch <= 32 && 100 * total_k < 85LL * batch * max_seqlen;
   const auto kernel = dump != nullptr ? attention_kernel<true, false> : by_length ? attention_kernel<false, true> : attention_kernel<false, false>;

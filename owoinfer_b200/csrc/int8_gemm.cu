@@ -190,7 +190,8 @@ __host__ __device__ constexpr int out_warp_bytes(Epi e) { return e == Epi::kSitu
 // kSplit > 1: a cluster of kSplit such tiles' CTAs (pairs) works on ONE output tile, each on its part of K. When their MMAs
 // are done every CTA hands the others' columns of its int32 accumulator over through distributed shared memory (into the
 // ring, which is idle by then) and finishes its own kBN / kSplit columns: exact sums, so the same bits. For problems of so
-// few tiles that half of the SMs would idle; the sums through L2 instead had cost 8 to 17 us a launch, this costs 1 to 2.
+// few tiles that half of the SMs would idle; the sums through L2 instead had cost 8 to 17 us a launch, this costs 1.1 (clusters of two
+// tiles' CTAs) to 3.4 (of four, by pairs).
 template <int kBN, Epi kEpi, int kCtas, bool kW4 = false, int kSplit = 1>
 __global__ void __launch_bounds__(threads_of(kEpi, kBN, kW4), 1)
 int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
@@ -577,7 +578,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       __syncwarp();
       // Gated residual: the residual rows of the warp's first 64 columns are asked for ahead of the accumulator (and those
       // of the next 64 ahead of the work on these), so that their way from L2 is not part of a tile's last microseconds:
-      // 0.4 to 0.8 us of a launch from 297 to 1050 rows. (The W4A8 kernels have no registers left for it.)
+      // 0.4 to 0.8 us of a launch from 297 to 1050 rows. (The W4A8 kernels, held to 96
+      // registers by their threads and spilling already, have none left for it.)
       [[maybe_unused]] uint4 ahead_res[8];
       [[maybe_unused]] const auto fetch_residual = [&](int c0) {
         const int pcol = nt * kBN + c0 + 8 * (lane & 7), r0 = mt * (kBM * kCtas) + static_cast<int>(rank) * kBM + quarter * 32 + (lane >> 3);
@@ -1049,6 +1051,11 @@ struct TileCost {
 //   297 x 8192     22.1      27.2         16.4              19.2
 //   400 x 8192     22.3      27.1                           19.5
 //   400 x 12288    30.7      36.3                           24.2
+//   256 x 8192     22.2      27.0         16.1              19.0           16.7
+//   256 x 12288    30.3      36.4         20.4              23.9           19.6
+//   256 x 16384    38.7      45.7         25.1              28.9           22.2
+// and with 1024 columns 256 x 16384: 37.8, 44.8, 23.3, 27.7, 19.7. Over 702 problems (512 to 9216 columns, K 512 to 16384, 1 to 640
+// rows) the choice below takes as long as the best of all six within 0.1 % on average, and 8 % at worst (640 x 512, 4608 columns).
 struct TileChoice {
   int tile, split;
 };
