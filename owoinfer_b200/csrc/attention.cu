@@ -1727,12 +1727,15 @@ int attention_impl(const char* op, const b2_attention_options* o, const b2_view3
   // them (121 us; by length 107). Of nearly equal lengths it gains little, and finding the tile costs each CTA some loads and
   // shuffles. Over 256 mixes (2 to 32 sequences, the longest 300 to 3000, 6 and 24 heads) whole calls by length took, by how full
   // batch x longest was: to 0.7 0.955 of batch order, to 0.8 0.97, to 0.86 0.99, to 0.93 0.998, above 1.005 to 1.012. (The one mix of
-  // those below the line that loses more than 3 %: 2400 + 3000 + 1800 keys, 6 heads, 86 us, by length 94.) It also keeps the
-  // empty CTAs of a generous max_seqlen out from between the full ones (4 x 1000 keys, 4 heads, max_seqlen 4000: 40 us, by length
-  // 36). The flat grid has no more CTAs than the query rows can fill tiles: with one for every tile up to max_seqlen the search of
-  // the empty ones takes 32 x 100 keys from 61 to 74 us at a max_seqlen of 1000 and from 468 to 840 at 16384.
+  // those below the line that loses more than 3 %: 2400 + 3000 + 1800 keys, 6 heads, 86 us, by length 94.) Where batch order
+  // has no more CTAs than there are SMs none waits for a place and the search is all loss: 1.7 % over 562 calls, at worst 13.3 us ->
+  // 14.7; from 148 to 300 CTAs by length gains 2 to 3 %, above that 4 to 24 %. It also keeps the empty CTAs of a generous
+  // max_seqlen out from between the full ones (4 x 1000 keys, 4 heads, max_seqlen 4000: 40 us, by length 36). The flat grid has no
+  // more CTAs than the query rows can fill tiles: with one for every tile up to max_seqlen the search of the empty ones takes
+  // 32 x 100 keys from 61 to 74 us at a max_seqlen of 1000 and from 468 to 840 at 16384.
   const std::int64_t most_tiles = std::min<std::int64_t>(static_cast<std::int64_t>(a.q_tiles) * batch, (total_q + (kTileQ - 1LL) * batch) / kTileQ) * heads;
-  const bool by_length = dump == nullptr && batch > 1 && batch <= 32 && 100 * total_k < 85LL * batch * max_seqlen;
+  const bool by_length = dump == nullptr && batch > 1 && batch <= 32 && 100 * total_k < 85LL * batch * max_seqlen &&
+                         static_cast<std::int64_t>(a.q_tiles) * batch * heads > sm_count();
   const auto kernel = dump != nullptr ? attention_kernel<true, false> : by_length ? attention_kernel<false, true> : attention_kernel<false, false>;
   if (const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
       e != cudaSuccess) {

@@ -266,9 +266,11 @@ def test_attention_of_a_batch_is_that_of_its_sequences(ops, lens, keys):
 @pytest.mark.parametrize("heads,lens,keys,longest,by_length", [
     (64, [300, 64, 700, 129], None, 700, True), (64, [1, 0, 257, 40], [513, 70, 64, 900], 900, True), (12, [130] + [40] * 31, None, 130, True),
     (12, [129] * 31, None, 16384, True), (64, [128, 1, 129, 1], None, 5000, True), (64, [1] * 32, None, 512, True), (64, [0, 128, 0, 513], None, 513, True),
-    (64, [200] + [33] * 33, None, 200, False), (3, [300, 64, 700, 129], None, 700, True), (1, [130, 2], None, 4096, True), (64, [300, 290], None, 300, False)])
+    (64, [200] + [33] * 33, None, 200, False), (7, [300, 64, 700, 129], None, 700, True), (3, [130, 2], None, 4096, True), (64, [300, 290], None, 300, False),
+    (3, [300, 64, 700, 129], None, 700, False), (1, [130, 2], None, 4096, False)])
 def test_attention_by_length_reaches_every_tile(ops, heads, lens, keys, longest, by_length):
-    """Sequences of different lengths are handed out longest first, up to 32 of them; else in batch order. The flat grid has to
+    """Sequences of different lengths are handed out longest first, up to 32 of them and where batch order has more CTAs than there
+    are SMs; else in batch order. The flat grid has to
     reach the last tile whatever the lengths leave of each tile."""
     keys = keys or lens
     q = torch.randn((sum(lens), heads, 128), device="cuda", generator=_gen(5)).bfloat16()
